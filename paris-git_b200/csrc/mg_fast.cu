@@ -44,7 +44,7 @@ __host__ __device__ inline int nu_at(int L, int nu, int nuc, int cf, int ct) {
 // x_new of a relaxed cell: the Gauss-Seidel value g, over-relaxed by w
 template <typename T>
 __device__ inline T relax(T g, T x0, T w) {
-    return w == (T)1 ? g : x0 + w * (g - x0);
+    return w == (T)1 ? g : fma(w, g - x0, x0);
 }
 
 template <typename T>
@@ -187,6 +187,7 @@ __global__ void k_fast_prolong(const LV<T> f, const LV<T> c) {
 static inline dim3 row_grid(long n0, int n1, int n2) { return dim3(div_up(n0, 128), n1, n2); }
 
 #include "mg_sweep.cuh"
+#include "mg_sweep_col.cuh"
 #include "mg_sweep_tma.cuh"
 #include "mg_sweep4.cuh"
 #include "mg_sweep_rs.cuh"
@@ -948,7 +949,7 @@ static int fast_alloc(paris_ctx* c) {
         // the fused sweep stages 16-byte row chunks and pairs cells by parity
         l.x2 = nullptr;
         bool fusable = l.N >= kFusedCells && l.N > kCoarseCells && l.n[0] % 4 == 0 && l.n[1] % 2 == 0 &&
-                       l.n[2] % 2 == 0 && L < nl - 1;
+                       l.n[2] % 2 == 0 && L < nl - 1 && l.N < 1L << 32;
         if (fusable) PARIS_CUDA_TRY(c, cudaMalloc(&l.x2, l.N * sizeof(T)));
         l.pairs = fusable && pairs_wanted();
         l.rs = fusable && std::is_same<T, float>::value && (rs_levels() == 2 || (rs_levels() == 1 && L == 0));
@@ -974,16 +975,16 @@ static int fast_coefs(paris_ctx* c) {
     return PARIS_OK;
 }
 
-// Planes per block of the fused sweep: enough blocks for one wave of resident
-// blocks, at least 4 planes per block (2 where that leaves fewer blocks than
-// SMs).
-template <class Cfg, bool M, typename T>
-static int sweep_chunk_cfg(paris_ctx* c, const FastLevel<T>& l) {
-    constexpr size_t smem = sweep2_smem_cfg<Cfg, M>();
+// Planes per block of the merged-phase sweep: enough blocks for one wave of
+// resident blocks, at least 4 planes per block (2 where that leaves fewer
+// blocks than SMs).
+template <class Cfg>
+static int sweep_merged_chunk(paris_ctx* c, const FastLevel<float>& l) {
+    constexpr size_t smem = sweep2_smem_cfg<Cfg>();
     static int per_sm = 0;   // resident blocks per SM (the same on every B200)
     if (!per_sm) {
-        cudaFuncSetAttribute(k_rb_sweep2_cfg<Cfg, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep2_cfg<Cfg, M>, Cfg::NT, smem) !=
+        cudaFuncSetAttribute(k_rb_sweep2_cfg<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep2_cfg<Cfg>, Cfg::NT, smem) !=
                 cudaSuccess || per_sm < 1)
             per_sm = 1;
     }
@@ -995,20 +996,16 @@ static int sweep_chunk_cfg(paris_ctx* c, const FastLevel<T>& l) {
     if (nbz < 1) nbz = 1;
     return (int)div_up(l.n[2], nbz);
 }
-template <typename T>
-static int sweep_chunk(paris_ctx* c, const FastLevel<T>& l) {
-    return sweep_chunk_cfg<typename SwGeo<T>::Cfg, false>(c, l);
-}
 
 // the merged-phase sweep of an FP32 level with configuration Cfg
 template <class Cfg>
 static int sweep_merged(paris_ctx* c, const FastLevel<float>& l, const char* label, const float* xin, float* xout,
                         const float* xc, int first, double* bx_part, int* bx_blocks) {
-    const int zc = sweep_chunk_cfg<Cfg, true>(c, l);
+    const int zc = sweep_merged_chunk<Cfg>(c, l);
     dim3 grid(div_up(l.n[0], Cfg::TX), div_up(l.n[1], Cfg::TY), div_up(l.n[2], zc));
     if (bx_part && (long)grid.x * grid.y * grid.z > kRedBlocks) bx_part = nullptr;
-    auto* const kern = &k_rb_sweep2_cfg<Cfg, true>;
-    constexpr size_t smem = sweep2_smem_cfg<Cfg, true>();
+    auto* const kern = &k_rb_sweep2_cfg<Cfg>;
+    constexpr size_t smem = sweep2_smem_cfg<Cfg>();
     PARIS_LAUNCH_N(c, kname<float>(label), l.N, kern, grid, Cfg::NT, smem, view(l), xin, xout, xc, c->bnd, first, zc,
                    bx_part);
     if (bx_part && bx_blocks) *bx_blocks = (int)(grid.x * grid.y * grid.z);
@@ -1034,12 +1031,70 @@ static int sweep_tma_chunk(paris_ctx* c, const FastLevel<float>& l) {
     return (int)div_up(l.n[2], nbz);
 }
 
-// bx_part: also write the per-block partials of b.x (see k_rb_sweep2_cfg);
+// Launch geometry of the column sweep with configuration C on level l: tiles
+// as wide as the grid where its chunks fit a staged row, else equal tiles with
+// one ring chunk on either side; planes per block (even) so that the blocks
+// fill whole waves of the C::MINB x nsm resident ones with long chunks (a
+// chunk takes about three planes' time before its first output).
+template <class C>
+static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l) {
+    const int n0 = l.n[0], n2 = l.n[2], V = C::VEC;
+    SwColGeo g;
+    if (n0 / V <= C::PITCH) {
+        g.W = n0;
+        g.H = 0;
+    } else {
+        const int t = (int)div_up(n0, (C::PITCH - 2) * V);
+        g.W = (int)div_up(div_up(n0, t), V) * V;
+        g.H = V;
+    }
+    g.lanes = (g.W + 2 * g.H) / V;
+    const long tiles = (long)div_up(n0, g.W) * div_up(l.n[1], C::TY), slots = (long)C::MINB * c->nsm;
+    double best = -1.0;
+    g.zc = n2;
+    for (int zc = 2; zc <= n2; zc += 2) {
+        const long blocks = tiles * div_up(n2, zc), waves = (blocks + slots - 1) / slots;
+        const double eff = (double)tiles * n2 / (double)(waves * slots * (zc + 3));
+        if (eff > best) {
+            best = eff;
+            g.zc = zc;
+        }
+    }
+    return g;
+}
+
+template <class C, bool ZERO, bool CORR>
+static int sweep_col_launch(paris_ctx* c, const char* label, const FastLevel<typename C::T>& l,
+                            const typename C::T* xin, typename C::T* xout, const typename C::T* xc, int first,
+                            double* bx_part, int* bx_blocks) {
+    static bool set = false;   // (the same value by every thread)
+    if (!set) {
+        PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k_rb_sweep_col<C, ZERO, CORR>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+        set = true;
+    }
+    const SwColGeo g = sweep_col_geo<C>(c, l);
+    const dim3 grid(div_up(l.n[0], g.W), div_up(l.n[1], C::TY), div_up(l.n[2], g.zc));
+    if (bx_part && (long)grid.x * grid.y * grid.z > kRedBlocks) bx_part = nullptr;
+    auto* const kern = &k_rb_sweep_col<C, ZERO, CORR>;
+    PARIS_LAUNCH_N(c, label, l.N, kern, grid, C::NT, C::SMEM, view(l), xin, xout, xc, c->bnd, first, g, bx_part);
+    if (bx_part && bx_blocks) *bx_blocks = (int)(grid.x * grid.y * grid.z);
+    return PARIS_OK;
+}
+
+template <class C>
+static int sweep_col(paris_ctx* c, const char* label, const FastLevel<typename C::T>& l, const typename C::T* xin,
+                     typename C::T* xout, const typename C::T* xc, int first, double* bx_part, int* bx_blocks) {
+    if (!xin) return sweep_col_launch<C, true, false>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
+    if (xc) return sweep_col_launch<C, false, true>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
+    return sweep_col_launch<C, false, false>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
+}
+
+// bx_part: also write the per-block partials of b.x (see k_rb_sweep_col);
 // *bx_blocks receives their count (0 when this form of the sweep cannot)
 template <typename T>
 static int sweep_fused(paris_ctx* c, int L, const FastLevel<T>& l, const T* xin, T* xout, const T* xc, int first,
                        double* bx_part = nullptr, int* bx_blocks = nullptr) {
-    using Cfg = typename SwGeo<T>::Cfg;
     // level 0 streams from HBM; the lower levels are resident in L2
     const char* label = L > 0 ? "mg_sweep_lower" : (xin ? "mg_sweep" : "mg_sweep_zero");
     if (bx_blocks) *bx_blocks = 0;
@@ -1058,13 +1113,23 @@ static int sweep_fused(paris_ctx* c, int L, const FastLevel<T>& l, const T* xin,
         if (l.merged == 1) return sweep_merged<SwMCfg12>(c, l, label, xin, xout, xc, first, bx_part, bx_blocks);
         if (l.merged == 2) return sweep_merged<SwMCfg14>(c, l, label, xin, xout, xc, first, bx_part, bx_blocks);
     }
-    int zc = sweep_chunk<T>(c, l);
-    dim3 grid(div_up(l.n[0], Cfg::TX), div_up(l.n[1], Cfg::TY), div_up(l.n[2], zc));
-    if (bx_part && (long)grid.x * grid.y * grid.z > kRedBlocks) bx_part = nullptr;
-    PARIS_LAUNCH_N(c, kname<T>(label), l.N, k_rb_sweep2_cfg<Cfg>, grid, Cfg::NT,
-                   sweep_smem<T>(), view(l), xin, xout, xc, c->bnd, first, zc, bx_part);
-    if (bx_part && bx_blocks) *bx_blocks = (int)(grid.x * grid.y * grid.z);
-    return PARIS_OK;
+    const int chunks = l.n[0] * (int)sizeof(T) / 16;
+    const char* name = kname<T>(label);
+#define SWEEP_COL(P, TY, D, MINB) \
+    return sweep_col<SwColCfg<T, P, TY, D, MINB>>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks)
+    // Rows of up to 16 and 32 chunks, and of 49 to 64 and (FP32) 97 to 128, as
+    // whole rows: no ring columns, and a warp's lanes lie in rows of one
+    // parity.  Other rows are cut into tiles of up to 14 output chunks.
+    // Measured us per sweep (B200), this form / the two-phase form it replaced:
+    // FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 256^3 87 / 138, 512x256x128 114 /
+    // 138, 320x192x160 (cut) 72 / 89; FP64 64^3 9.8 / 10.8, 128^3 30 / 44,
+    // 256x128x128 (cut) 69 / 78, 192x192x96 (cut) 53 / 60.
+    if (chunks <= 16) SWEEP_COL(16, 6, sizeof(T) == 4 ? 3 : 2, 4);
+    if (chunks <= 32) SWEEP_COL(32, (sizeof(T) == 4 ? 6 : 4), 2, (sizeof(T) == 4 ? 2 : 3));
+    if (chunks > 48 && chunks <= 64) SWEEP_COL(64, (sizeof(T) == 4 ? 7 : 8), 2, 1);
+    if (sizeof(T) == 4 && chunks > 96 && chunks <= 128) SWEEP_COL(128, 4, 1, 1);
+    SWEEP_COL(16, 10, 2, 3);
+#undef SWEEP_COL
 }
 
 // planes per block of the fused-restriction sweep: one wave of resident

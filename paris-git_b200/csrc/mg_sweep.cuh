@@ -1,24 +1,22 @@
-// mg_sweep.cuh -- fused red-black Gauss-Seidel sweep of the B200 multigrid
-// (included by mg_fast.cu after LV<T>).
+// mg_sweep.cuh -- fused red-black Gauss-Seidel sweep of the B200 multigrid with
+// scalar shared-memory operands, and the update shared by every form of the
+// sweep (included by mg_fast.cu after LV<T>).  The solver's own form is
+// k_rb_sweep_col (mg_sweep_col.cuh); this one, one barrier per pair of planes,
+// is opt-in (PARIS_SWEEP_MERGED) and gives the same iterates to the bit.
 //
 // One full sweep (colour F = `first`, then the other colour S) in one pass
 // over memory.  A block owns a TX x TY column of cells and marches up a
-// chunk of planes with a wavefront, two planes per step:
-//   step (f0, f1 = f0+1):  F at planes f0 and f1 on the tile plus a one-cell
-//             ring (from the old iterate), then S at planes f0-1 and f0 on the
-//             tile (from the new F values of the planes around them); planes
-//             f0-1 and f0 are then final and stored.
-// Planes of the iterate (tile + two-cell ring) and of the coefficients are
-// staged in shared memory with 16-byte cp.async, D steps ahead of their use,
-// so that enough bytes are in flight per SM to cover the HBM latency; each
-// array is read from HBM once per sweep (the ring re-reads hit L2).  The
-// iterate is read from `xin` (nullptr: zero) and written to `xout`, never in
-// place, so blocks never see each other's new values and the sweep computes
-// the two colour passes of k_fast_smooth (in FP64 exactly; in FP32 with the
-// update arithmetic of SwUpd<float>).  With `xc`, the coarse-grid
-// correction (injection from the level below) is added to the iterate as it
-// arrives, fetched into registers one step ahead.  Ring-buffer slots rotate
-// with the step.
+// chunk of planes with a wavefront, two planes per step.  Planes of the iterate
+// (tile + two-cell ring) and of the coefficients are staged in shared memory
+// with 16-byte cp.async, D steps ahead of their use, so that enough bytes are
+// in flight per SM to cover the HBM latency; each array is read from HBM once
+// per sweep (the ring re-reads hit L2).  The iterate is read from `xin`
+// (nullptr: zero) and written to `xout`, never in place, so blocks never see
+// each other's new values and the sweep computes the two colour passes of
+// k_fast_smooth (in FP64 exactly; in FP32 with the update arithmetic of
+// SwUpd<float>).  With `xc`, the coarse-grid correction (injection from the
+// level below) is added to the iterate as it arrives, fetched into registers
+// one step ahead.  Ring-buffer slots rotate with the step.
 //
 // With bx_part, the sweep also sums b x over the cells it stores (in FP64) and
 // writes one partial per block: on the last sweep of a V-cycle on the finest
@@ -37,28 +35,10 @@ struct SwCfg {
     using type = T_;
     static constexpr int TY = TY_, D = D_, NT = NT_, MINB = MINB_, TX = TX_;
 };
-// the configurations the solver uses
-template <typename T>
-struct SwGeo;
-template <>
-struct SwGeo<float> {
-    using Cfg = SwCfg<float, 16, 1, 320, 2>;   // 32x16 tiles, two planes staged ahead, two blocks per SM
-};
-template <>
-struct SwGeo<double> {
-    using Cfg = SwCfg<double, 8, 1, 256, 2>;   // 32x8 tiles: two blocks per SM within shared memory
-};
 // the merged-phase form (FP32, opt-in): its deeper rings fit two blocks per
 // SM with 32x12 or 32x14 tiles
 using SwMCfg12 = SwCfg<float, 12, 1, 256, 2>;
 using SwMCfg14 = SwCfg<float, 14, 1, 288, 2>;
-
-template <class C, bool M = false>
-static constexpr size_t sweep2_smem_cfg();
-template <typename T>
-static constexpr size_t sweep_smem() {
-    return sweep2_smem_cfg<typename SwGeo<T>::Cfg>();
-}
 
 // VEC/2 coarse values of a staged chunk, loaded together
 template <typename T, int N>
@@ -98,17 +78,18 @@ __device__ inline int sw_wrap(int a, int n, int per) {
     return a < 0 ? a + n : a;
 }
 
-// The Gauss-Seidel update x = s / d of one cell.  FP32 (the inner cycle of
-// the mixed solver): the sums as trees of depth three instead of chains of
-// seven dependent adds, and the fast division (two ulps); the smoother only
-// has to reduce the error, the FP64 outer loop keeps the residual exact.
-// FP64: the sums in the order of A1..A6 and the IEEE division.
+// The Gauss-Seidel update x = s / d of one cell, with the fused multiply-adds
+// written out so that every form of the sweep rounds alike.  FP32 (the inner
+// cycle of the mixed solver): the sums as trees of depth three, and the fast
+// division (two ulps); the smoother only has to reduce the error, the
+// FP64 outer loop keeps the residual exact.  FP64: the sums in the order of
+// A1..A6 and the IEEE division.
 template <typename T>
 struct SwUpd {
     __device__ static inline bool apply(T a1, T a2, T a3, T a4, T a5, T a6, T x1, T x2, T x3, T x4, T x5, T x6, T b,
                                         T x0, T w, T& out) {
-        T d = a1 + a2 + a3 + a4 + a5 + a6;
-        T s = a1 * x1 + a2 * x2 + a3 * x3 + a4 * x4 + a5 * x5 + a6 * x6 + b;
+        const T d = a1 + a2 + a3 + a4 + a5 + a6;
+        const T s = fma(a6, x6, fma(a5, x5, fma(a4, x4, fma(a3, x3, fma(a1, x1, a2 * x2))))) + b;
         if (d > (T)0) { out = relax(s / d, x0, w); return true; }
         return false;
     }
@@ -119,7 +100,7 @@ struct SwUpd<float> {
                                         float x2, float x3, float x4, float x5, float x6, float b, float x0, float w,
                                         float& out) {
         const float d = ((a1 + a2) + (a3 + a4)) + (a5 + a6);
-        const float s = ((a1 * x1 + a2 * x2) + (a3 * x3 + a4 * x4)) + ((a5 * x5 + a6 * x6) + b);
+        const float s = (fmaf(a1, x1, a2 * x2) + fmaf(a3, x3, a4 * x4)) + (fmaf(a5, x5, a6 * x6) + b);
         if (d > 0.f) { out = relax(__fdividef(s, d), x0, w); return true; }
         return false;
     }
@@ -133,20 +114,15 @@ __device__ inline int sw_add(int s, int d, int S) {
 }
 
 // ---------------------------------------------------------------------------
-// Step s works on f0 = z0-1+2s and f1 = f0+1; the barriers and the ring
-// bookkeeping of a step are shared by two planes, and each thread has two
-// independent updates per phase.  Live planes: iterate f0-2..f1+1,
-// coefficients f0-1..f1, cz f0-2..f1, each plus 2D staged ahead.
-//
-// M (merged phases): the second colour of step s-1 (planes f0-3, f0-2) and
-// the first colour of step s (planes f0, f0+1) run in one phase between two
-// barriers.  They touch disjoint cells: the first colour writes its cells of
-// planes f0, f0+1 and reads second-colour cells of planes f0-1..f0+2, which
-// the second colour of step s-1 does not write; that one writes its cells of
-// planes f0-3, f0-2 and reads first-colour cells of planes f0-4..f0-1, final
-// since the phases before.  One barrier per step instead of two, for a ring
-// two planes deeper (iterate f0-4..f0+2, coefficients f0-3..f0+1, cz
-// f0-4..f0+1, plus 2D staged ahead).
+// Step s works on f0 = z0-1+2s and f0+1: the second colour of step s-1 (planes
+// f0-3, f0-2) and the first colour of step s (planes f0, f0+1) run in one phase
+// between two barriers.  They touch disjoint cells: the first colour writes its
+// cells of planes f0, f0+1 and reads second-colour cells of planes f0-1..f0+2,
+// which the second colour of step s-1 does not write; that one writes its cells
+// of planes f0-3, f0-2 and reads first-colour cells of planes f0-4..f0-1, final
+// since the phases before.  Live planes with M: iterate f0-4..f0+2,
+// coefficients f0-3..f0+1, cz f0-4..f0+1, plus 2D staged ahead; two planes
+// fewer each for the two-phase step of k_rb_sweep_tma (M false).
 template <class C, bool M = false>
 struct Sw2 {
     using T = typename C::type;
@@ -168,18 +144,18 @@ struct Sw2 {
     static_assert(CH <= NT, "one chunk of each array per thread");
 };
 
-template <class C, bool M>
+template <class C>
 static constexpr size_t sweep2_smem_cfg() {
-    return sizeof(typename C::type) * (size_t)Sw2<C, M>::RP * Sw2<C, M>::SLOTS;
+    return sizeof(typename C::type) * (size_t)Sw2<C, true>::RP * Sw2<C, true>::SLOTS;
 }
 
-template <class C, bool M = false>
+template <class C>
 __global__ void __launch_bounds__(C::NT, C::MINB)
     k_rb_sweep2_cfg(const LV<typename C::type> v, const typename C::type* __restrict__ xin,
                     typename C::type* __restrict__ xout, const typename C::type* __restrict__ xc, const Bnd B,
                     int first, int zc, double* __restrict__ bx_part) {
     using T = typename C::type;
-    using G = Sw2<C, M>;
+    using G = Sw2<C, true>;
     constexpr int NT = G::NT;
     constexpr int RX = G::RX, RP = G::RP, TY = G::TY, VEC = G::VEC;
     extern __shared__ __align__(16) unsigned char sw_raw[];
@@ -365,75 +341,27 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         fetch_coarse(0, f0 + 3);
         fetch_coarse(1, f0 + 4);
     };
-    if constexpr (M) {
-        // slot of plane k >= kb - S in a ring of S slots
-        auto sl = [&](int k, int S) { return (k - kb + S) % S; };
-        auto X = [&](int k) { return rx_ + sl(k, G::XS) * RP; };
-        auto CX = [&](int k) { return rcx + sl(k, G::CS) * RP; };
-        auto CY = [&](int k) { return rcy + sl(k, G::CS) * RP; };
-        auto BB = [&](int k) { return rb + sl(k, G::CS) * RP; };
-        auto CZ = [&](int k) { return rcz + sl(k, G::ZS) * RP; };
-        for (int f0 = z0 - 1; f0 <= z1 + 2; f0 += 2) {
-            cp_async_wait_newest<G::D - 1>();
-            if (xc) coarse_step(f0);
-            __syncthreads();
-            stage_x(f0 + 2 * G::D + 1, sl(f0 + 2 * G::D + 1, G::XS));
-            stage_x(f0 + 2 * G::D + 2, sl(f0 + 2 * G::D + 2, G::XS));
-            stage_c(f0 + 2 * G::D, sl(f0 + 2 * G::D, G::CS), sl(f0 + 2 * G::D, G::ZS), false);
-            stage_c(f0 + 2 * G::D + 1, sl(f0 + 2 * G::D + 1, G::CS), sl(f0 + 2 * G::D + 1, G::ZS), false);
-            cp_async_commit();
-            s_at(f0 - 3, X(f0 - 3), X(f0 - 4), X(f0 - 2), CX(f0 - 3), CY(f0 - 3), BB(f0 - 3), CZ(f0 - 3), CZ(f0 - 4));
-            s_at(f0 - 2, X(f0 - 2), X(f0 - 3), X(f0 - 1), CX(f0 - 2), CY(f0 - 2), BB(f0 - 2), CZ(f0 - 2), CZ(f0 - 3));
-            if (f0 <= z1) f_at(f0, X(f0), X(f0 - 1), X(f0 + 1), CX(f0), CY(f0), BB(f0), CZ(f0), CZ(f0 - 1));
-            if (f0 + 1 <= z1)
-                f_at(f0 + 1, X(f0 + 1), X(f0), X(f0 + 2), CX(f0 + 1), CY(f0 + 1), BB(f0 + 1), CZ(f0 + 1), CZ(f0));
-        }
-    }
-    // ring positions of plane f0-2 (iterate, cz) and f0-1 (coefficients),
-    // advanced by two each step (plane z0-2 sits in slot 0 of every ring)
-    int xb = G::XS - 1, cb = 0, zb = G::ZS - 1;
-    for (int f0 = z0 - 1; f0 <= z1 && !M; f0 += 2) {
+    // slot of plane k >= kb - S in a ring of S slots
+    auto sl = [&](int k, int S) { return (k - kb + S) % S; };
+    auto X = [&](int k) { return rx_ + sl(k, G::XS) * RP; };
+    auto CX = [&](int k) { return rcx + sl(k, G::CS) * RP; };
+    auto CY = [&](int k) { return rcy + sl(k, G::CS) * RP; };
+    auto BB = [&](int k) { return rb + sl(k, G::CS) * RP; };
+    auto CZ = [&](int k) { return rcz + sl(k, G::ZS) * RP; };
+    for (int f0 = z0 - 1; f0 <= z1 + 2; f0 += 2) {
         cp_async_wait_newest<G::D - 1>();
-        if (xc) {   // the iterate planes that arrived: group 0's, then two per step
-            if (f0 == z0 - 1) {
-                for (int k = z0 - 2; k <= z0 + 1; k++) {
-                    fetch_coarse(0, k);
-                    add_coarse(0, k);
-                }
-            } else {
-                if (f0 + 1 <= z1 + 1) add_coarse(0, f0 + 1);   // planes above z1+1 are never staged
-                if (f0 + 2 <= z1 + 1) add_coarse(1, f0 + 2);
-            }
-            fetch_coarse(0, f0 + 3);
-            fetch_coarse(1, f0 + 4);
-        }
+        if (xc) coarse_step(f0);
         __syncthreads();
-        // slots of planes f0+2D+1, f0+2D+2 (iterate) and f0+2D, f0+2D+1
-        // (coefficients): those of planes f0-4, f0-3 and f0-3, f0-2
-        stage_x(f0 + 2 * G::D + 1, sw_add(xb, -2, G::XS));
-        stage_x(f0 + 2 * G::D + 2, sw_add(xb, -1, G::XS));
-        stage_c(f0 + 2 * G::D, sw_add(cb, -2, G::CS), sw_add(zb, -2, G::ZS), false);
-        stage_c(f0 + 2 * G::D + 1, sw_add(cb, -1, G::CS), sw_add(zb, -1, G::ZS), false);
+        stage_x(f0 + 2 * G::D + 1, sl(f0 + 2 * G::D + 1, G::XS));
+        stage_x(f0 + 2 * G::D + 2, sl(f0 + 2 * G::D + 2, G::XS));
+        stage_c(f0 + 2 * G::D, sl(f0 + 2 * G::D, G::CS), sl(f0 + 2 * G::D, G::ZS), false);
+        stage_c(f0 + 2 * G::D + 1, sl(f0 + 2 * G::D + 1, G::CS), sl(f0 + 2 * G::D + 1, G::ZS), false);
         cp_async_commit();
-        // iterate planes f0-2 .. f0+2, coefficient planes f0-1 .. f0+1, cz f0-2 .. f0+1
-        T* const xm2 = rx_ + xb * RP;
-        T* const xm1 = rx_ + sw_add(xb, 1, G::XS) * RP;
-        T* const x0p = rx_ + sw_add(xb, 2, G::XS) * RP;
-        T* const x1p = rx_ + sw_add(xb, 3, G::XS) * RP;
-        T* const x2p = rx_ + sw_add(xb, 4, G::XS) * RP;
-        const int c0 = sw_add(cb, 1, G::CS), c1 = sw_add(cb, 2, G::CS);
-        const T* const zm2 = rcz + zb * RP;
-        const T* const zm1 = rcz + sw_add(zb, 1, G::ZS) * RP;
-        const T* const z0p = rcz + sw_add(zb, 2, G::ZS) * RP;
-        const T* const z1p = rcz + sw_add(zb, 3, G::ZS) * RP;
-        f_at(f0, x0p, xm1, x1p, rcx + c0 * RP, rcy + c0 * RP, rb + c0 * RP, z0p, zm1);
-        if (f0 + 1 <= z1) f_at(f0 + 1, x1p, x0p, x2p, rcx + c1 * RP, rcy + c1 * RP, rb + c1 * RP, z1p, z0p);
-        __syncthreads();
-        s_at(f0 - 1, xm1, xm2, x0p, rcx + cb * RP, rcy + cb * RP, rb + cb * RP, zm1, zm2);
-        s_at(f0, x0p, xm1, x1p, rcx + c0 * RP, rcy + c0 * RP, rb + c0 * RP, z0p, zm1);
-        xb = sw_add(xb, 2, G::XS);
-        cb = sw_add(cb, 2, G::CS);
-        zb = sw_add(zb, 2, G::ZS);
+        s_at(f0 - 3, X(f0 - 3), X(f0 - 4), X(f0 - 2), CX(f0 - 3), CY(f0 - 3), BB(f0 - 3), CZ(f0 - 3), CZ(f0 - 4));
+        s_at(f0 - 2, X(f0 - 2), X(f0 - 3), X(f0 - 1), CX(f0 - 2), CY(f0 - 2), BB(f0 - 2), CZ(f0 - 2), CZ(f0 - 3));
+        if (f0 <= z1) f_at(f0, X(f0), X(f0 - 1), X(f0 + 1), CX(f0), CY(f0), BB(f0), CZ(f0), CZ(f0 - 1));
+        if (f0 + 1 <= z1)
+            f_at(f0 + 1, X(f0 + 1), X(f0), X(f0 + 2), CX(f0 + 1), CY(f0 + 1), BB(f0 + 1), CZ(f0 + 1), CZ(f0));
     }
     cp_async_wait_all_groups();
     if (bx_part) {   // b.x of the block: one partial per block, in launch order
