@@ -244,7 +244,7 @@ extern "C" int paris_gpu_finalize(paris_handle_t c) {
                     (void*)c->rhs, (void*)c->A, (void*)c->red_part, (void*)c->fast_r64,
                     (void*)c->fast_d64, (void*)c->fast_q64,
                     (void*)c->vflux, (void*)c->mixlist, (void*)c->mixsegn, (void*)c->kflag, (void*)c->st_list,
-                    (void*)c->st_count, (void*)c->debris_count, (void*)c->cg_scal, (void*)c->adj, (void*)c->stats_part, (void*)c->stats_out, (void*)c->mom_tab,
+                    (void*)c->st_count, (void*)c->debris_count, (void*)c->ref_bar, (void*)c->cg_scal, (void*)c->adj, (void*)c->stats_part, (void*)c->stats_out, (void*)c->mom_tab,
                     (void*)c->mc_tmp, (void*)c->mc_tmp2, (void*)c->mc_work, (void*)c->mc_fv, (void*)c->mc_flag,
                     (void*)c->mc_cg})
         free_ptr(p);
@@ -258,7 +258,7 @@ extern "C" int paris_gpu_finalize(paris_handle_t c) {
     }
     if (c->s_h2d) cudaStreamDestroy(c->s_h2d);
     if (c->s_d2h) cudaStreamDestroy(c->s_d2h);
-    for (auto& l : c->ref) { free_ptr(l.K); free_ptr(l.p); free_ptr(l.e); }
+    for (auto& l : c->ref) { free_ptr(l.K); free_ptr(l.p); free_ptr(l.e); free_ptr(l.q); }
     mg_fast_free_maps(c);
     for (auto& l : c->fl32) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); }
     for (auto& l : c->fl64) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); }

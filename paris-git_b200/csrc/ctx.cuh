@@ -15,6 +15,7 @@ struct RefLevel {
     double* K;   // 8*N
     double* p;   // pMG
     double* e;   // EMG
+    double* q;   // beta / K7
 };
 
 // One level of the B200 multigrid: face coefficients (east/north/top of each
@@ -80,6 +81,7 @@ struct paris_ctx {
     // multigrid hierarchies
     int ref_lmg = 0;
     std::vector<RefLevel> ref;     // index 1..LMG
+    unsigned* ref_bar = nullptr;   // grid barrier of the cycle kernel
     int fast_nl = 0;
     int fast_nuc = 0, fast_cf = 1, fast_ct = 0;   // sweeps on the levels fast_cf..fast_ct (0: nu1/nu2), set by each solve
     std::vector<FastLevel<float>> fl32;

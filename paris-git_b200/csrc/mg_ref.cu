@@ -14,55 +14,237 @@ struct LvlDims {
     long N;
 };
 
-__device__ inline double nbr(const double* __restrict__ x, const LvlDims& d, const Bnd& B, int i, int j, int k) {
-    if (i < 0 || i >= d.n0) { if (!B.per[0]) return 0.0; i = i < 0 ? i + d.n0 : i - d.n0; }
-    if (j < 0 || j >= d.n1) { if (!B.per[1]) return 0.0; j = j < 0 ? j + d.n1 : j - d.n1; }
-    if (k < 0 || k >= d.n2) { if (!B.per[2]) return 0.0; k = k < 0 ? k + d.n2 : k - d.n2; }
-    return x[cidx(d.n0, d.n1, i, j, k)];
-}
-
-// RedBlackRelax, one colour: (i+j+k+color) even cells (local indices).
-__global__ void k_ref_relax(const double* __restrict__ K, double* __restrict__ p, const LvlDims d, const Bnd B,
-                            double beta, int color) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    int h0 = (d.n0 + 1) / 2;
-    if (t >= (long)h0 * d.n1 * d.n2) return;
-    int ih = (int)(t % h0), j = (int)((t / h0) % d.n1), k = (int)(t / ((long)h0 * d.n1));
-    int i = 2 * ih + ((j + k + color) & 1);
-    if (i >= d.n0) return;
-    long m = cidx(d.n0, d.n1, i, j, k);
-    long N = d.N;
-    p[m] = (1.0 - beta) * p[m] +
-           beta / K[6 * N + m] *
-               (K[0 * N + m] * nbr(p, d, B, i - 1, j, k) + K[1 * N + m] * nbr(p, d, B, i + 1, j, k) +
-                K[2 * N + m] * nbr(p, d, B, i, j - 1, k) + K[3 * N + m] * nbr(p, d, B, i, j + 1, k) +
-                K[4 * N + m] * nbr(p, d, B, i, j, k - 1) + K[5 * N + m] * nbr(p, d, B, i, j, k + 1) + K[7 * N + m]);
-}
-
 __device__ inline double powabs(double r, int norm) {
     double a = fabs(r);
     return norm == 2 ? a * a : (norm == 1 ? a : pow(a, (double)norm));
 }
 
-// get_residual: K8 <- K8 - K7 p + sum K_n p_n (in place); optional sum |r|^norm
-__global__ void k_ref_get_residual(double* __restrict__ K, const double* __restrict__ p, const LvlDims d,
-                                   const Bnd B, int norm, double* part) {
+// ---- MG_iteration in one kernel ---------------------------------------------
+// One cycle is some seventy dependent passes over levels of 64^3 cells and less:
+// as launches of their own they took 5.9 us each, whatever their size, 530 us
+// per iteration at 64^3 (its residual and host wait included); as one kernel
+// 245 us, bound by the latency of a pass (a barrier over the grid and one round
+// of loads from L2).  Here the whole cycle is one cooperative kernel, a block
+// per SM, with a barrier over the grid after each pass; levels of at most
+// kRefOneBlock cells are worked by block 0 alone, with block barriers.  Passes
+// that need no barrier between them are one: the first colour from a zero
+// iterate also zeroes the other; the residual and its restriction; the
+// prolonged correction is read from the coarse iterate where it is used, never
+// stored; the sum with the correction and the residual after it.
+// All level extents are powers of two (init_MG), so cells come from shifts.
+// Values that other blocks write within the kernel are read past L1 (__ldcg).
+static constexpr int kRefThreads = 1024;
+static constexpr int kRefOneBlock = 512;   // (16^3 over the grid: its colour pass is two cells a thread in one block)
+static constexpr int kRefMaxLevels = 16;
+static constexpr long kRefSpin = 1L << 24;   // polls of a barrier before it gives up (seconds)
+
+struct RefLvl {
+    int b0, b1, b2;   // log2 of the extents
+    double *K, *p, *e;
+    const double* q;   // beta / K7, formed once per solve
+};
+struct RefCycle {
+    RefLvl l[kRefMaxLevels + 1];   // 1..lmg
+    int lmg, nrelax, sym;
+    double beta;
+};
+
+__device__ inline int ref_cell(const RefLvl& l, int i, int j, int k) { return (((k << l.b1) + j) << l.b0) + i; }
+
+// the six neighbours' values f(i,j,k), 0 beyond a wall: loaded at the wrapped
+// index without a branch, so that all of them are in flight together
+template <typename F>
+__device__ inline void ref_nbrs(const RefLvl& l, const Bnd& B, int i, int j, int k, F f, double x[6]) {
+    const int e0 = (1 << l.b0) - 1, e1 = (1 << l.b1) - 1, e2 = (1 << l.b2) - 1;
+    x[0] = f((i - 1) & e0, j, k);
+    x[1] = f((i + 1) & e0, j, k);
+    x[2] = f(i, (j - 1) & e1, k);
+    x[3] = f(i, (j + 1) & e1, k);
+    x[4] = f(i, j, (k - 1) & e2);
+    x[5] = f(i, j, (k + 1) & e2);
+    if (!B.per[0]) {
+        if (i == 0) x[0] = 0.0;
+        if (i == e0) x[1] = 0.0;
+    }
+    if (!B.per[1]) {
+        if (j == 0) x[2] = 0.0;
+        if (j == e1) x[3] = 0.0;
+    }
+    if (!B.per[2]) {
+        if (k == 0) x[4] = 0.0;
+        if (k == e2) x[5] = 0.0;
+    }
+}
+
+// RedBlackRelax, one colour: (i+j+k+color) even cells (local indices); zero:
+// the iterate is zero and is written whole
+__device__ inline void ref_relax(const RefLvl& l, double* x, const Bnd& B, double beta, int color, bool zero, int t0,
+                                 int st) {
+    const int N = 1 << (l.b0 + l.b1 + l.b2), h = l.b0 - 1;
+    const double* K = l.K;
+    auto f = [&](int i, int j, int k) { return __ldcg(x + ref_cell(l, i, j, k)); };
+    for (int t = t0; t < N / 2; t += st) {
+        const int j = (t >> h) & ((1 << l.b1) - 1), k = t >> (h + l.b1);
+        const int i = 2 * (t & ((1 << h) - 1)) + ((j + k + color) & 1), m = ref_cell(l, i, j, k);
+        const double k7 = __ldcg(K + 7L * N + m);
+        if (zero) {
+            x[m] = (1.0 - beta) * 0.0 + l.q[m] * (0.0 + k7);
+            x[m ^ 1] = 0.0;
+            continue;
+        }
+        double y[6];
+        ref_nbrs(l, B, i, j, k, f, y);
+        x[m] = (1.0 - beta) * __ldcg(x + m) +
+               l.q[m] * (K[m] * y[0] + K[1L * N + m] * y[1] + K[2L * N + m] * y[2] + K[3L * N + m] * y[3] +
+                         K[4L * N + m] * y[4] + K[5L * N + m] * y[5] + k7);
+    }
+}
+
+// get_residual of cell m with the iterate f: K8 <- K8 - K7 x + sum K_n x_n
+template <typename F>
+__device__ inline double ref_residual(const RefLvl& l, const Bnd& B, int i, int j, int k, int m, F f) {
+    const int N = 1 << (l.b0 + l.b1 + l.b2);
+    double* K = l.K;
+    double y[6];
+    ref_nbrs(l, B, i, j, k, f, y);
+    const double r = __ldcg(K + 7L * N + m) - K[6L * N + m] * f(i, j, k) + K[m] * y[0] + K[1L * N + m] * y[1] +
+                     K[2L * N + m] * y[2] + K[3L * N + m] * y[3] + K[4L * N + m] * y[4] + K[5L * N + m] * y[5];
+    K[7L * N + m] = r;
+    return r;
+}
+
+// The blocks of the grid meet: monotonic arrivals at bar[0].  A block that
+// polls too long raises bar[1] and *err, and every block leaves the kernel.
+__device__ inline bool ref_grid_sync(unsigned* bar, unsigned& want, int* err) {
+    __shared__ int gone;
+    want += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        gone = 0;
+        long polls = 0;
+        unsigned v;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (++polls > kRefSpin || *(volatile unsigned*)(bar + 1)) {
+                gone = 1;
+                atomicExch(bar + 1, 1u);
+                *err = 1;
+                break;
+            }
+        } while (v < want);
+        __threadfence();
+    }
+    __syncthreads();
+    return gone == 0;
+}
+
+// MG_iteration, MGsolver.f90:253-320
+__global__ void __launch_bounds__(kRefThreads, 1) k_ref_cycle(const RefCycle C, const Bnd B, unsigned* bar, int* err) {
+    unsigned want = 0;
+    const int gt = blockIdx.x * kRefThreads + threadIdx.x, gs = gridDim.x * kRefThreads;
+    const double beta = C.beta;
+    auto size = [](const RefLvl& l) { return 1 << (l.b0 + l.b1 + l.b2); };
+    int q = 1;   // levels 1..q are worked by block 0 alone
+    while (q < C.lmg && size(C.l[q + 1]) <= kRefOneBlock) q++;
+    // the passes of a level on the way down: relaxed from zero, its residual,
+    // and the coarse right-hand side; in the order of coarse_from_fine
+    // (k1 fastest, then j1, i1)
+    auto restrict_ = [&](const RefLvl& l, const RefLvl& c, int t0, int st) {
+        const int Nc = size(c);
+        auto f = [&](int i, int j, int k) { return __ldcg(l.p + ref_cell(l, i, j, k)); };
+        for (int t = t0; t < Nc; t += st) {
+            const int i = t & ((1 << c.b0) - 1), j = (t >> c.b0) & ((1 << c.b1) - 1), k = t >> (c.b0 + c.b1);
+            double s = 0.0;
+#pragma unroll 2
+            for (int u = 0; u < 8; u++) {
+                const int I = 2 * i + (u >> 2), J = 2 * j + ((u >> 1) & 1), Kk = 2 * k + (u & 1);
+                s = s + ref_residual(l, B, I, J, Kk, ref_cell(l, I, J, Kk), f) * 0.125;
+            }
+            c.K[7L * Nc + t] = s;
+        }
+    };
+    // the correction injected from the level below (sym_MG weights it by the
+    // just-zeroed correction): residual with it, and the iterate plus it
+    auto correct = [&](const RefLvl& l, const RefLvl& c, int t0, int st) {
+        const int N = size(l);
+        const double wt = C.sym ? 0.0 : 1.0;
+        auto f = [&](int i, int j, int k) { return wt * __ldcg(c.p + ref_cell(c, i >> 1, j >> 1, k >> 1)); };
+        for (int m = t0; m < N; m += st) {
+            const int i = m & ((1 << l.b0) - 1), j = (m >> l.b0) & ((1 << l.b1) - 1), k = m >> (l.b0 + l.b1);
+            ref_residual(l, B, i, j, k, m, f);
+            l.p[m] = __ldcg(l.p + m) + f(i, j, k);
+        }
+    };
+    // the iterate plus the relaxed correction e, and the residual with e
+    auto finish = [&](const RefLvl& l, int t0, int st) {
+        const int N = size(l);
+        auto f = [&](int i, int j, int k) { return __ldcg(l.e + ref_cell(l, i, j, k)); };
+        for (int m = t0; m < N; m += st) {
+            const int i = m & ((1 << l.b0) - 1), j = (m >> l.b0) & ((1 << l.b1) - 1), k = m >> (l.b0 + l.b1);
+            l.p[m] = __ldcg(l.p + m) + f(i, j, k);
+            ref_residual(l, B, i, j, k, m, f);
+        }
+    };
+#define REF_SYNC()                                    \
+    do {                                              \
+        if (one) __syncthreads();                     \
+        else if (!ref_grid_sync(bar, want, err)) return; \
+    } while (0)
+    for (int part = 0; part < 3; part++) {
+        // down the large levels; the small levels down and up (block 0); up the large levels
+        const bool one = part == 1;
+        const int t0 = one ? threadIdx.x : gt, st = one ? kRefThreads : gs;
+        if (!one || blockIdx.x == 0) {
+            const int hi = one ? q : C.lmg, low = one ? 2 : (q + 1 > 2 ? q + 1 : 2);
+            if (part < 2)
+                for (int L = hi; L >= low; L--) {
+                    const RefLvl& l = C.l[L];
+                    for (int r = 0; r < 2 * C.nrelax; r++) {
+                        ref_relax(l, l.p, B, beta, r & 1, r == 0, t0, st);
+                        REF_SYNC();
+                    }
+                    restrict_(l, C.l[L - 1], t0, st);
+                    REF_SYNC();
+                }
+            if ((one && q >= 2) || (part == 2 && q < 2)) {   // level 2 once more
+                for (int color = 0; color < 2; color++) {
+                    ref_relax(C.l[2], C.l[2].p, B, beta, color, false, t0, st);
+                    REF_SYNC();
+                }
+            }
+            if (part > 0)
+                for (int L = one ? 3 : (q + 1 > 3 ? q + 1 : 3); L <= hi; L++) {
+                    const RefLvl& l = C.l[L];
+                    correct(l, C.l[L - 1], t0, st);
+                    REF_SYNC();
+                    for (int r = 0; r < 2 * C.nrelax; r++) {
+                        ref_relax(l, l.e, B, beta, r & 1, r == 0, t0, st);
+                        REF_SYNC();
+                    }
+                    finish(l, t0, st);
+                    REF_SYNC();
+                }
+        }
+        if (one && !ref_grid_sync(bar, want, err)) return;
+    }
+#undef REF_SYNC
+}
+
+// K8 <- K8 - K7 p + sum K_n p_n on the finest level (initial residual) and its
+// sum |r|^norm
+__global__ void k_ref_initial_residual(const RefLvl l, const Bnd B, int norm, double* part) {
     __shared__ double sh[32];
     double s = 0.0;
-    long N = d.N;
-    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < N; m += (long)gridDim.x * blockDim.x) {
-        int i = (int)(m % d.n0), j = (int)((m / d.n0) % d.n1), k = (int)(m / ((long)d.n0 * d.n1));
-        double r = K[7 * N + m] - K[6 * N + m] * p[m] + K[0 * N + m] * nbr(p, d, B, i - 1, j, k) +
-                   K[1 * N + m] * nbr(p, d, B, i + 1, j, k) + K[2 * N + m] * nbr(p, d, B, i, j - 1, k) +
-                   K[3 * N + m] * nbr(p, d, B, i, j + 1, k) + K[4 * N + m] * nbr(p, d, B, i, j, k - 1) +
-                   K[5 * N + m] * nbr(p, d, B, i, j, k + 1);
-        K[7 * N + m] = r;
-        if (part) s += powabs(r, norm);
+    const int N = 1 << (l.b0 + l.b1 + l.b2);
+    auto f = [&](int i, int j, int k) { return l.p[ref_cell(l, i, j, k)]; };
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < N; m += gridDim.x * blockDim.x) {
+        const int i = m & ((1 << l.b0) - 1), j = (m >> l.b0) & ((1 << l.b1) - 1), k = m >> (l.b0 + l.b1);
+        s += powabs(ref_residual(l, B, i, j, k, m, f), norm);
     }
-    if (part) {
-        s = block_sum<256>(s, sh);
-        if (threadIdx.x == 0) part[blockIdx.x] = s;
-    }
+    s = block_sum<256>(s, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
 // compute_residual on the finest level with the caller's A and the ghosted p
@@ -70,17 +252,22 @@ __global__ void k_ref_compute_residual(const double* __restrict__ A, const doubl
                                        int norm, double* part) {
     __shared__ double sh[32];
     double s = 0.0;
-    long N = (long)L.n[0] * L.n[1] * L.n[2];
-    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < N; m += (long)gridDim.x * blockDim.x) {
-        int i = (int)(m % L.n[0]), j = (int)((m / L.n[0]) % L.n[1]), k = (int)(m / ((long)L.n[0] * L.n[1]));
-        long n = lidx(L, i, j, k);
+    const long N = (long)L.n[0] * L.n[1] * L.n[2];
+    ROWS_BEGIN(L.n[0], L.n[1], L.n[2])
+        const long m = cidx(L.n[0], L.n[1], i, j, k), n = lidx(L, i, j, k);
         double r = A[7 * N + m] - A[6 * N + m] * p[n] + A[0 * N + m] * p[n - 1] + A[1 * N + m] * p[n + 1] +
                    A[2 * N + m] * p[n - L.pitch] + A[3 * N + m] * p[n + L.pitch] +
                    A[4 * N + m] * p[n - L.plane] + A[5 * N + m] * p[n + L.plane];
         s += powabs(r, norm);
-    }
+    ROWS_END
     s = block_sum<256>(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    if (linear_tid() == 0) part[blockIdx.x] = s;
+}
+
+// beta / K7 of a level (RedBlackRelax divides in every pass; the same quotient)
+__global__ void k_ref_quotient(const double* __restrict__ K7, double* __restrict__ q, double beta, long N) {
+    const long m = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (m < N) q[m] = beta / K7[m];
 }
 
 // fill_coefficients: 0.125*(sum of the 8 children in the Fortran order)
@@ -100,53 +287,11 @@ __global__ void k_ref_fill_coef(const double* __restrict__ Kf, const LvlDims f, 
     Kc[comp * c.N + m] = 0.125 * s;
 }
 
-// coarse_from_fine: Ac8 = 0; Ac8 += Af8*0.125 with k1 fastest, then j1, i1
-__global__ void k_ref_coarse_from_fine(const double* __restrict__ Kf, const LvlDims f, double* __restrict__ Kc,
-                                       const LvlDims c) {
-    long m = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (m >= c.N) return;
-    int i = (int)(m % c.n0), j = (int)((m / c.n0) % c.n1), k = (int)(m / ((long)c.n0 * c.n1));
-    const double* F = Kf + 7 * f.N;
-    double s = 0.0;
-    for (int i1 = 0; i1 < 2; i1++)
-        for (int j1 = 0; j1 < 2; j1++)
-            for (int k1 = 0; k1 < 2; k1++) s = s + F[cidx(f.n0, f.n1, 2 * i + i1, 2 * j + j1, 2 * k + k1)] * 0.125;
-    Kc[7 * c.N + m] = s;
-}
-
-// coarse_fine_interp: injection (sym_MG: weights |pf| of the children)
-__global__ void k_ref_interp(double* __restrict__ ef, const LvlDims f, const double* __restrict__ pc,
-                             const LvlDims c, int sym) {
-    long m = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (m >= c.N) return;
-    int i = (int)(m % c.n0), j = (int)((m / c.n0) % c.n1), k = (int)(m / ((long)c.n0 * c.n1));
-    double v = pc[m];
-    long q[8];
-    int t = 0;
-    for (int dk = 0; dk < 2; dk++)
-        for (int dj = 0; dj < 2; dj++)
-            for (int di = 0; di < 2; di++) q[t++] = cidx(f.n0, f.n1, 2 * i + di, 2 * j + dj, 2 * k + dk);
-    if (sym) {
-        double rt = fabs(ef[q[0]]) + fabs(ef[q[1]]) + fabs(ef[q[2]]) + fabs(ef[q[3]]) + fabs(ef[q[4]]) +
-                    fabs(ef[q[5]]) + fabs(ef[q[6]]) + fabs(ef[q[7]]) + 1.e-15;
-        for (int s = 0; s < 8; s++) ef[q[s]] = fabs(ef[q[s]]) / rt * v;
-    } else {
-        for (int s = 0; s < 8; s++) ef[q[s]] = v;
-    }
-}
-
-__global__ void k_ref_add(double* __restrict__ a, const double* __restrict__ b, long N) {
-    long m = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (m < N) a[m] = a[m] + b[m];
-}
-
 // pMG(LMG) <- p (interior) and p <- p + pMG(LMG)
 __global__ void k_ref_field_io(double* __restrict__ pf, double* __restrict__ pm, const Layout L, int add) {
-    long m = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long N = (long)L.n[0] * L.n[1] * L.n[2];
-    if (m >= N) return;
-    int i = (int)(m % L.n[0]), j = (int)((m / L.n[0]) % L.n[1]), k = (int)(m / ((long)L.n[0] * L.n[1]));
-    long n = lidx(L, i, j, k);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+    if (i >= L.n[0]) return;
+    const long m = cidx(L.n[0], L.n[1], i, j, k), n = lidx(L, i, j, k);
     if (add) pf[n] = pf[n] + pm[m];
     else pm[m] = pf[n];
 }
@@ -166,7 +311,7 @@ static int ref_alloc(paris_ctx* c) {
         while ((1 << (L + 1)) <= nd[a]) L++;
         lmg = L < lmg ? L : lmg;
     }
-    if (lmg < 2) return PARIS_BAD_ARGS;
+    if (lmg < 2 || lmg > kRefMaxLevels || c->N > 1L << 30) return PARIS_BAD_ARGS;
     c->ref_lmg = lmg;
     c->ref.resize(lmg + 1);
     for (int L = lmg; L >= 1; L--) {
@@ -176,50 +321,34 @@ static int ref_alloc(paris_ctx* c) {
         PARIS_CUDA_TRY(c, cudaMalloc(&l.K, 8 * l.N * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMalloc(&l.p, l.N * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMalloc(&l.e, l.N * sizeof(double)));
+        PARIS_CUDA_TRY(c, cudaMalloc(&l.q, l.N * sizeof(double)));
     }
     return PARIS_OK;
 }
 
-static int relax(paris_ctx* c, RefLevel& l, double* x, double beta) {
-    LvlDims d = dims(l);
-    long nt = (long)((d.n0 + 1) / 2) * d.n1 * d.n2;
-    PARIS_LAUNCH(c, k_ref_relax, div_up(nt, 256), 256, 0, l.K, x, d, c->bnd, beta, 0);
-    PARIS_LAUNCH(c, k_ref_relax, div_up(nt, 256), 256, 0, l.K, x, d, c->bnd, beta, 1);
-    return PARIS_OK;
+static int log2_of(int n) {
+    int b = 0;
+    while ((1 << (b + 1)) <= n) b++;
+    return b;
 }
 
-static int get_residual(paris_ctx* c, RefLevel& l, double* x) {
-    LvlDims d = dims(l);
-    unsigned g = div_up(d.N, 256);
-    if (g > 65535u) g = 65535u;
-    PARIS_LAUNCH(c, k_ref_get_residual, g, 256, 0, l.K, x, d, c->bnd, 2, (double*)nullptr);
-    return PARIS_OK;
+static RefLvl ref_level(const RefLevel& l) {
+    return RefLvl{log2_of(l.n[0]), log2_of(l.n[1]), log2_of(l.n[2]), l.K, l.p, l.e, l.q};
 }
 
-// MG_iteration, MGsolver.f90:253-320
-static int mg_iteration(paris_ctx* c, double beta, int nrelax, int sym) {
-    int lmg = c->ref_lmg;
-    for (int L = lmg; L >= 2; L--) {
-        RefLevel& l = c->ref[L];
-        PARIS_CUDA_TRY(c, cudaMemsetAsync(l.p, 0, l.N * sizeof(double), c->stream));
-        for (int r = 0; r < nrelax; r++) PARIS_CHECK(relax(c, l, l.p, beta));
-        PARIS_CHECK(get_residual(c, l, l.p));
-        RefLevel& lc = c->ref[L - 1];
-        PARIS_LAUNCH(c, k_ref_coarse_from_fine, div_up(lc.N, 256), 256, 0, l.K, dims(l), lc.K, dims(lc));
-    }
-    PARIS_CHECK(relax(c, c->ref[2], c->ref[2].p, beta));
-    for (int L = 3; L <= lmg; L++) {
-        RefLevel& l = c->ref[L];
-        RefLevel& lc = c->ref[L - 1];
-        PARIS_CUDA_TRY(c, cudaMemsetAsync(l.e, 0, l.N * sizeof(double), c->stream));
-        PARIS_LAUNCH(c, k_ref_interp, div_up(lc.N, 256), 256, 0, l.e, dims(l), lc.p, dims(lc), sym);
-        PARIS_CHECK(get_residual(c, l, l.e));
-        PARIS_LAUNCH(c, k_ref_add, div_up(l.N, 256), 256, 0, l.p, l.e, l.N);
-        PARIS_CUDA_TRY(c, cudaMemsetAsync(l.e, 0, l.N * sizeof(double), c->stream));
-        for (int r = 0; r < nrelax; r++) PARIS_CHECK(relax(c, l, l.e, beta));
-        PARIS_LAUNCH(c, k_ref_add, div_up(l.N, 256), 256, 0, l.p, l.e, l.N);
-        PARIS_CHECK(get_residual(c, l, l.e));
-    }
+// one cycle: a cooperative launch, so that all its blocks are resident
+static int mg_iteration(paris_ctx* c, const RefCycle& C) {
+    if (!c->ref_bar) PARIS_CUDA_TRY(c, cudaMalloc(&c->ref_bar, 2 * sizeof(unsigned)));
+    PARIS_CUDA_TRY(c, cudaMemsetAsync(c->ref_bar, 0, 2 * sizeof(unsigned), c->stream));
+    RefCycle a = C;
+    void* args[] = {&a, &c->bnd, &c->ref_bar, &c->err_dev};
+    const bool prof = prof_enabled(c);
+    if (prof) prof_begin(c, "k_ref_cycle", c->N);
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_ref_cycle, dim3(c->nsm), dim3(kRefThreads), args, 0,
+                                                      c->stream);
+    if (prof) prof_end(c);
+    c->launches++;
+    PARIS_CUDA_TRY(c, e);
     return PARIS_OK;
 }
 
@@ -233,23 +362,37 @@ int mg_ref_solve(paris_ctx* c, const paris_solve_opts* o, paris_solve_result* re
     for (int L = lmg - 1; L >= 1; L--)
         PARIS_LAUNCH(c, k_ref_fill_coef, div_up(8 * c->ref[L].N, 256), 256, 0, c->ref[L + 1].K, dims(c->ref[L + 1]),
                      c->ref[L].K, dims(c->ref[L]));
+    for (int L = lmg; L >= 2; L--)
+        PARIS_LAUNCH(c, k_ref_quotient, div_up(c->ref[L].N, 256), 256, 0, c->ref[L].K + 6 * c->ref[L].N, c->ref[L].q,
+                     o->beta, c->ref[L].N);
     double* p = c->fld[PARIS_FIELD_P];
-    PARIS_LAUNCH(c, k_ref_field_io, div_up(lf.N, 256), 256, 0, p, lf.p, c->L, 0);
-    PARIS_LAUNCH(c, k_ref_get_residual, red_grid(c, k_ref_get_residual, 256), 256, 0, lf.K, lf.p, dims(lf), c->bnd, o->norm, c->red_part);
+    PARIS_LAUNCH(c, k_ref_field_io, dim3(div_up(c->d.nx, 128), c->d.ny, c->d.nz), 128, 0, p, lf.p, c->L, 0);
+    PARIS_LAUNCH(c, k_ref_initial_residual, red_grid(c, k_ref_initial_residual, 256), 256, 0, ref_level(lf), c->bnd,
+                 o->norm, c->red_part);
     double s;
     PARIS_CHECK(ctx_reduce_finish(c, 1, &s));
     double nxyz = (double)c->d.nx * (double)c->d.ny * (double)c->d.nz;
     double tres2 = s / nxyz;
     res->res0 = o->norm == 2 ? sqrt(tres2) : tres2;
     PARIS_CUDA_TRY(c, cudaMemsetAsync(lf.p, 0, lf.N * sizeof(double), c->stream));
-    int nrelax = c->d.nrelax > 0 ? c->d.nrelax : 3;
+    RefCycle C;
+    for (int L = 1; L <= lmg; L++) C.l[L] = ref_level(c->ref[L]);
+    C.lmg = lmg;
+    C.nrelax = c->d.nrelax > 0 ? c->d.nrelax : 3;
+    C.sym = c->d.sym_mg;
+    C.beta = o->beta;
     int it;
     for (it = 1; it <= o->maxit; it++) {
-        PARIS_CHECK(mg_iteration(c, o->beta, nrelax, c->d.sym_mg));
-        PARIS_LAUNCH(c, k_ref_field_io, div_up(lf.N, 256), 256, 0, p, lf.p, c->L, 1);
+        PARIS_CHECK(mg_iteration(c, C));
+        PARIS_LAUNCH(c, k_ref_field_io, dim3(div_up(c->d.nx, 128), c->d.ny, c->d.nz), 128, 0, p, lf.p, c->L, 1);
         PARIS_CHECK(ctx_ghost_fill(c, p));
-        PARIS_LAUNCH(c, k_ref_compute_residual, red_grid(c, k_ref_compute_residual, 256), 256, 0, c->A, p, c->L, o->norm, c->red_part);
+        PARIS_LAUNCH(c, k_ref_compute_residual, red_grid(c, k_ref_compute_residual, 256), kRowBlock, 0, c->A, p, c->L, o->norm, c->red_part);
         PARIS_CHECK(ctx_reduce_finish(c, 1, &s));
+        if (*c->err_host) {
+            *c->err_host = 0;
+            ctx_set_error(c, "a barrier of the reference multigrid cycle ran out");
+            return PARIS_CUDA_ERROR;
+        }
         tres2 = s / nxyz;
         if (o->norm == 2) tres2 = sqrt(tres2);
         if (tres2 != tres2) {
