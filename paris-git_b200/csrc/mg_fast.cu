@@ -8,7 +8,8 @@
 //   the colours reversed after the coarse correction (symmetric cycle).
 // The inner cycle runs in T = float (mixed) or double; the outer loop is FP64:
 // defect correction p += V(b - A p), or CG preconditioned by the V-cycle.
-// Levels at or below kCoarseCells cells run in one single-block kernel.
+// Levels at or below kCoarseCells cells run in one single-block kernel; a
+// coarsest level above that is relaxed by the colour passes.
 #include <stdlib.h>
 #include <string.h>
 #include <type_traits>
@@ -19,12 +20,11 @@ static constexpr long kCoarseCells = 4096;   // 16^3
 static constexpr int kMaxLevels = 16;
 static constexpr int kCoarseSweeps = 8;
 static constexpr long kWarpCells = 64;   // coarse levels of at most 4^3 cells run in one warp
-static constexpr long kFusedCells = 1L << 15;
+static constexpr long kFusedCells = 1L << 15;   // levels of at least 32^3 cells can take the fused sweep
 // device-side scalars of the CG loop (paris_ctx::cg_scal): r.z of the two
 // latest preconditioned residuals (alternating), d.q, and r.r, sum |r|, r.z_old
 // from the update
 static constexpr int kScRZ0 = 0, kScDQ = 2, kScRR = 3, kScRZold = 5;
-static constexpr size_t kCoarseSmemMax = 227 * 1024;   // opt-in shared memory per block   // levels of at least 64^3 cells use the fused sweep
 
 template <typename T>
 struct LV {
@@ -82,27 +82,6 @@ __device__ inline void smooth_cell(const LV<T>& v, const Bnd& B, int i, int j, i
     T d = a1 + a2 + a3 + a4 + a5 + a6;
     T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + v.b[m];
     if (d > (T)0) v.x[m] = relax(s / d, v.omega != (T)1 ? v.x[m] : (T)0, v.omega);
-}
-
-template <typename T>
-__device__ inline T resid_cell(const LV<T>& v, const Bnd& B, int i, int j, int k) {
-    long m = cidx(v.n0, v.n1, i, j, k);
-    T a1, a3, a5, xw, xe, xs, xn, xb, xt;
-    west_coefs(v, B, i, j, k, m, a1, a3, a5);
-    T a2 = v.cx[m], a4 = v.cy[m], a6 = v.cz[m];
-    nbrs(v, v.x, B, i, j, k, m, xw, xe, xs, xn, xb, xt);
-    T d = a1 + a2 + a3 + a4 + a5 + a6;
-    return v.b[m] - d * v.x[m] + a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt;
-}
-
-// coarse rhs = mean of the 8 fine residuals
-template <typename T>
-__device__ inline void restrict_cell(const LV<T>& f, const LV<T>& c, const Bnd& B, int i, int j, int k) {
-    T s = 0;
-    for (int dk = 0; dk < 2; dk++)
-        for (int dj = 0; dj < 2; dj++)
-            for (int di = 0; di < 2; di++) s += resid_cell(f, B, 2 * i + di, 2 * j + dj, 2 * k + dk);
-    c.b[cidx(c.n0, c.n1, i, j, k)] = (T)0.125 * s;
 }
 
 // grid (ceil(n/128), n1, n2), block 128: one thread per cell of the colour
@@ -164,7 +143,7 @@ __global__ void __launch_bounds__(128) k_fast_restrict2(const LV<T> f, const LV<
     }
     T s = (T)0;
     if (ok) {
-        // the fine cell i0, then i0+1 (the arithmetic of resid_cell)
+        // the fine cell i0, then i0+1
         T d = a1w + CX.x + CYS.x + CY.x + CZB.x + CZ.x;
         const T rA = BB.x - d * X.x + a1w * xw + CX.x * X.y + CYS.x * XS.x + CY.x * XN.x + CZB.x * XB.x + CZ.x * XT.x;
         d = CX.x + CX.y + CYS.y + CY.y + CZB.y + CZ.y;
@@ -192,54 +171,6 @@ static inline dim3 row_grid(long n0, int n1, int n2) { return dim3(div_up(n0, 12
 #include "mg_sweep4.cuh"
 #include "mg_sweep_rs.cuh"
 
-// 32-bit forms of smooth_cell / resid_cell / restrict_cell for the levels of
-// the single-block coarse cycle (at most a few thousand cells): the same
-// operations on the same values, with int instead of long index arithmetic.
-template <typename T>
-__device__ inline void nbrs32(const LV<T>& v, const T* x, const Bnd& B, int i, int j, int k, int m, T& a1, T& a3,
-                              T& a5, T& xw, T& xe, T& xs, T& xn, T& xb, T& xt) {
-    const int n0 = v.n0, n1 = v.n1, n2 = v.n2, sy = n0, sz = n0 * n1;
-    a1 = i > 0 ? v.cx[m - 1] : (B.per[0] ? v.cx[m + n0 - 1] : (T)0);
-    a3 = j > 0 ? v.cy[m - sy] : (B.per[1] ? v.cy[m + sy * (n1 - 1)] : (T)0);
-    a5 = k > 0 ? v.cz[m - sz] : (B.per[2] ? v.cz[m + sz * (n2 - 1)] : (T)0);
-    xw = i > 0 ? x[m - 1] : (B.per[0] ? x[m + n0 - 1] : (T)0);
-    xe = i < n0 - 1 ? x[m + 1] : (B.per[0] ? x[m - (n0 - 1)] : (T)0);
-    xs = j > 0 ? x[m - sy] : (B.per[1] ? x[m + sy * (n1 - 1)] : (T)0);
-    xn = j < n1 - 1 ? x[m + sy] : (B.per[1] ? x[m - sy * (n1 - 1)] : (T)0);
-    xb = k > 0 ? x[m - sz] : (B.per[2] ? x[m + sz * (n2 - 1)] : (T)0);
-    xt = k < n2 - 1 ? x[m + sz] : (B.per[2] ? x[m - sz * (n2 - 1)] : (T)0);
-}
-
-template <typename T>
-__device__ inline void smooth_cell32(const LV<T>& v, const Bnd& B, int i, int j, int k) {
-    const int m = i + v.n0 * (j + v.n1 * k);
-    T a1, a3, a5, xw, xe, xs, xn, xb, xt;
-    nbrs32(v, v.x, B, i, j, k, m, a1, a3, a5, xw, xe, xs, xn, xb, xt);
-    T a2 = v.cx[m], a4 = v.cy[m], a6 = v.cz[m];
-    T d = a1 + a2 + a3 + a4 + a5 + a6;
-    T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + v.b[m];
-    if (d > (T)0) v.x[m] = relax(s / d, v.omega != (T)1 ? v.x[m] : (T)0, v.omega);
-}
-
-template <typename T>
-__device__ inline T resid_cell32(const LV<T>& v, const Bnd& B, int i, int j, int k) {
-    const int m = i + v.n0 * (j + v.n1 * k);
-    T a1, a3, a5, xw, xe, xs, xn, xb, xt;
-    nbrs32(v, v.x, B, i, j, k, m, a1, a3, a5, xw, xe, xs, xn, xb, xt);
-    T a2 = v.cx[m], a4 = v.cy[m], a6 = v.cz[m];
-    T d = a1 + a2 + a3 + a4 + a5 + a6;
-    return v.b[m] - d * v.x[m] + a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt;
-}
-
-template <typename T>
-__device__ inline void restrict_cell32(const LV<T>& f, const LV<T>& c, const Bnd& B, int i, int j, int k) {
-    T s = 0;
-    for (int dk = 0; dk < 2; dk++)
-        for (int dj = 0; dj < 2; dj++)
-            for (int di = 0; di < 2; di++) s += resid_cell32(f, B, 2 * i + di, 2 * j + dj, 2 * k + dk);
-    c.b[i + c.n0 * (j + c.n1 * k)] = (T)0.125 * s;
-}
-
 // t / d for 0 <= t, d < 2^22 (exact): a float estimate within one of the
 // quotient, corrected
 __device__ inline int div_small(int t, int d, float rd) {
@@ -250,127 +181,15 @@ __device__ inline int div_small(int t, int d, float rd) {
     return q;
 }
 
-// The V-cycle from level L0 down to the coarsest, in one block, on copies of
-// those levels in shared memory: the coefficients of every level and the
-// right-hand side of level L0 are loaded, the cycle runs, and the iterate of
-// level L0 is written back.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_fast_coarse_cycle(const LVSet<T> G, int L0, int nl, const Bnd B, int nu1,
-                                                            int nu2, int nuc, int cf, int ct, int in_smem) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    extern __shared__ __align__(16) unsigned char cc_raw[];
-    __shared__ LV<T> S[kMaxLevels];   // level views, read by value in every phase
-    if (tid == 0) {
-        T* p = reinterpret_cast<T*>(cc_raw);
-        for (int L = L0; L < nl; L++) {
-            LV<T> l = G.l[L];
-            if (in_smem) {
-                T* cx = p;
-                l.cx = cx; l.cy = cx + l.N; l.cz = cx + 2 * l.N;
-                l.b = cx + 3 * l.N;
-                l.x = cx + 4 * l.N;
-                p = cx + 5 * l.N;
-            }
-            S[L] = l;
-        }
-    }
-    __syncthreads();
-    if (in_smem) {
-        for (int L = L0; L < nl; L++) {
-            const LV<T> g = G.l[L], l = S[L];
-            T* cx = const_cast<T*>(l.cx);
-            T* cy = const_cast<T*>(l.cy);
-            T* cz = const_cast<T*>(l.cz);
-            for (int t = tid; t < (int)g.N; t += nt) {
-                cx[t] = g.cx[t]; cy[t] = g.cy[t]; cz[t] = g.cz[t];
-                if (L == L0) l.b[t] = g.b[t];
-            }
-        }
-        __syncthreads();
-    }
-    // 32-bit index arithmetic throughout (levels here have at most a few
-    // thousand cells; 64-bit division would dominate every phase).  Levels of
-    // at most kWarpCells cells are worked by warp 0 alone with warp barriers.
-    const int lane = tid & 31;
-    auto smooth = [&](const LV<T> v, int color, bool warp) {
-        const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
-        const int h0 = (v.n0 + 1) >> 1, hn = h0 * v.n1;
-        const int tot = hn * v.n2;
-        const float rhn = 1.0f / (float)hn, rh0 = 1.0f / (float)h0;
-        for (int t = t0; t < tot; t += st) {
-            int k = div_small(t, hn, rhn), r = t - k * hn;
-            int j = div_small(r, h0, rh0), ih = r - j * h0;
-            int i = 2 * ih + ((j + k + color) & 1);
-            if (i < v.n0) smooth_cell32(v, B, i, j, k);
-        }
-        if (warp) __syncwarp();
-        else __syncthreads();
-    };
-    auto down = [&](int L, bool warp) {   // zero, pre-smooth and restrict level L, or solve the coarsest
-        const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
-        const LV<T> v = S[L];
-        for (int t = t0; t < (int)v.N; t += st) v.x[t] = (T)0;
-        if (warp) __syncwarp();
-        else __syncthreads();
-        if (L == nl - 1) {
-            for (int s = 0; s < kCoarseSweeps; s++) { smooth(v, 0, warp); smooth(v, 1, warp); }
-            for (int s = 0; s < kCoarseSweeps; s++) { smooth(v, 1, warp); smooth(v, 0, warp); }
-            return;
-        }
-        for (int s = 0; s < nu_at(L, nu1, nuc, cf, ct); s++) { smooth(v, 0, warp); smooth(v, 1, warp); }
-        const LV<T> c = S[L + 1];
-        const int cn = c.n0 * c.n1;
-        const float rcn = 1.0f / (float)cn, rc0 = 1.0f / (float)c.n0;
-        for (int t = t0; t < (int)c.N; t += st) {
-            int k = div_small(t, cn, rcn), r = t - k * cn;
-            int j = div_small(r, c.n0, rc0), i = r - j * c.n0;
-            restrict_cell32(v, c, B, i, j, k);
-        }
-        if (warp) __syncwarp();
-        else __syncthreads();
-    };
-    auto up = [&](int L, bool warp) {     // prolong into level L and post-smooth it
-        const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
-        const LV<T> v = S[L], c = S[L + 1];
-        const int fn = v.n0 * v.n1;
-        const float rfn = 1.0f / (float)fn, rf0 = 1.0f / (float)v.n0;
-        for (int t = t0; t < (int)v.N; t += st) {
-            int k = div_small(t, fn, rfn), r = t - k * fn;
-            int j = div_small(r, v.n0, rf0), i = r - j * v.n0;
-            v.x[t] += c.x[(i >> 1) + c.n0 * ((j >> 1) + c.n1 * (k >> 1))];
-        }
-        if (warp) __syncwarp();
-        else __syncthreads();
-        for (int s = 0; s < nu_at(L, nu2, nuc, cf, ct); s++) { smooth(v, 1, warp); smooth(v, 0, warp); }
-    };
-    int Lw = L0;   // first level worked by warp 0
-    while (Lw < nl && S[Lw].N > kWarpCells) Lw++;
-    for (int L = L0; L < Lw; L++) down(L, false);
-    if (Lw < nl) {
-        if (tid < 32) {
-            for (int L = Lw; L < nl; L++) down(L, true);
-            for (int L = nl - 2; L >= Lw; L--) up(L, true);
-        }
-        __syncthreads();
-    }
-    for (int L = min(Lw, nl - 1) - 1; L >= L0; L--) up(L, false);
-    if (in_smem) {
-        const LV<T> g = G.l[L0], l = S[L0];
-        for (int t = tid; t < (int)g.N; t += nt) g.x[t] = l.x[t];
-    }
-}
-
 // ---- the coarse cycle in shared memory ------------------------------------
-// The same cycle as k_fast_coarse_cycle, with every level of at most 16^3
-// cells held in the block's shared memory and addressed by element offsets
-// from one shared array (shared-memory loads rather than generic ones), the
-// neighbours of a cell taken branch-free (the wrapped or clamped index always
+// The V-cycle from level L0 (at most 16^3 cells) down to the coarsest in one
+// block, every level held in the block's shared memory and addressed by element
+// offsets from one shared array (shared-memory loads rather than generic ones),
+// the neighbours of a cell taken branch-free (the wrapped or clamped index always
 // loaded, the value dropped at a wall), the cell indices of each thread
 // decomposed once per pass, and the restriction split into a pass over the
 // fine cells (their residuals into a scratch array) and one over the coarse
-// cells (the 8 residuals summed in the order restrict_cell32 sums them).
-// The arithmetic of every update, residual and sum is that of
-// smooth_cell32 / resid_cell32 / restrict_cell32.
+// cells (the 8 residuals summed with i fastest).
 struct CcLvl {
     int n0, n1, n2, N;
     int cx, cy, cz, b, x;   // element offsets of the arrays in shared memory
@@ -573,7 +392,7 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
     }
 }
 
-// shared memory of k_fast_coarse_cycle: five arrays per level from L0 down
+// shared memory of k_coarse_cycle_smem: five arrays per level from L0 down
 template <typename T>
 static size_t coarse_smem(const std::vector<FastLevel<T>>& lv, int L0) {
     size_t n = 0;
@@ -1117,17 +936,20 @@ static int sweep_fused(paris_ctx* c, int L, const FastLevel<T>& l, const T* xin,
     const char* name = kname<T>(label);
 #define SWEEP_COL(P, TY, D, MINB) \
     return sweep_col<SwColCfg<T, P, TY, D, MINB>>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks)
-    // Rows of up to 16 and 32 chunks, and of 49 to 64 and (FP32) 97 to 128, as
-    // whole rows: no ring columns, and a warp's lanes lie in rows of one
-    // parity.  Other rows are cut into tiles of up to 14 output chunks.
+    // Rows of up to 64 chunks, and (FP32) of 97 to 128, as whole rows: no ring
+    // columns, and a warp's lanes lie in rows of one parity.  Other rows are cut
+    // into tiles of up to 14 output chunks.
     // Measured us per sweep (B200), this form / the two-phase form it replaced:
-    // FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 256^3 87 / 138, 512x256x128 114 /
-    // 138, 320x192x160 (cut) 72 / 89; FP64 64^3 9.8 / 10.8, 128^3 30 / 44,
-    // 256x128x128 (cut) 69 / 78, 192x192x96 (cut) 53 / 60.
+    // FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 184x180x100 30 / 38, 256^3 87 / 138,
+    // 512x256x128 114 / 138, 320x192x160 (cut) 72 / 89; FP64 64^3 9.8 / 10.8,
+    // 96x64x80 13.3 / 15.3, 128^3 30 / 44, 144x176x56 (cut) 28 / 38, 256x128x128
+    // (cut) 69 / 78, 208x112x32 (cut) 19.5 / 19.2.
     if (chunks <= 16) SWEEP_COL(16, 6, sizeof(T) == 4 ? 3 : 2, 4);
     if (chunks <= 32) SWEEP_COL(32, (sizeof(T) == 4 ? 6 : 4), 2, (sizeof(T) == 4 ? 2 : 3));
-    if (chunks > 48 && chunks <= 64) SWEEP_COL(64, (sizeof(T) == 4 ? 7 : 8), 2, 1);
-    if (sizeof(T) == 4 && chunks > 96 && chunks <= 128) SWEEP_COL(128, 4, 1, 1);
+    if (chunks <= 48) SWEEP_COL(48, (sizeof(T) == 4 ? 5 : 8), (sizeof(T) == 4 ? 1 : 2), (sizeof(T) == 4 ? 2 : 1));
+    if (chunks <= 64) SWEEP_COL(64, (sizeof(T) == 4 ? 7 : 8), 2, 1);
+    if constexpr (sizeof(T) == 4)
+        if (chunks > 96 && chunks <= 128) SWEEP_COL(128, 4, 1, 1);
     SWEEP_COL(16, 10, 2, 3);
 #undef SWEEP_COL
 }
@@ -1253,15 +1075,21 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_LAUNCH_N(c, kname<T>("mg_restrict"), l.N, k_fast_restrict2<T>,
                            dim3(div_up(cv.n0, 32), cv.n1, cv.n2), dim3(32, 4), 0, view_x(l, cur[L]), cv, c->bnd);
     }
-    LVSet<T> S;
-    for (int L = 0; L < nl; L++) S.l[L] = view(lv[L]);
-    // the levels run in shared memory when they fit (always for L0 <= 16^3)
-    // (the shared-memory cycle adds a scratch array of the largest restricted level)
-    const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
-    size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
-    const int in_smem = csm <= kCoarseSmemMax ? 1 : 0;
-    if (!in_smem) csm = 0;
-    if (in_smem) {
+    if (lv[Lc].N > kCoarseCells) {   // the coarsest, too large for a block
+        const LV<T> v = view(lv[Lc]);
+        PARIS_CUDA_TRY(c, cudaMemsetAsync(v.x, 0, v.N * sizeof(T), c->stream));
+        for (int s = 0; s < 4 * kCoarseSweeps; s++) {
+            const int color = s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1);
+            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2),
+                           128, 0, v, c->bnd, color);
+        }
+    } else {
+        LVSet<T> S;
+        for (int L = 0; L < nl; L++) S.l[L] = view(lv[L]);
+        // the levels and a scratch array of the largest restricted one fit the
+        // shared memory (at most 219 KB, FP64 from 16^3 down)
+        const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
+        const size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
         static size_t csm_set = 0;   // opt-in size set for this instantiation
         if (csm > csm_set) {
             PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k_coarse_cycle_smem<T>,
@@ -1270,9 +1098,6 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
         }
         PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, k_coarse_cycle_smem<T>, 1, 1024, csm, S, Lc, nl,
                        c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
-    } else {
-        PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, k_fast_coarse_cycle<T>, 1, 1024, 0, S, Lc, nl,
-                       c->bnd, nu1_, nu2_, nuc, cf, ct, 0);
     }
     cur[Lc] = lv[Lc].x;
     for (int L = Lc - 1; L >= 0; L--) {
