@@ -35,76 +35,109 @@ struct StArgs {
 
 __device__ inline double* Hidx(const StArgs& a, int index1) { return a.H + (long)(index1 - 1) * a.L.total; }
 
-__device__ inline long at(const StArgs& a, const int c[3]) {
-    return lidx(a.L, c[0], c[1], c[2]);
-}
-
 // Fortran index of interior-relative coordinate c: c + ng + 1
 __device__ inline double fidx(const StArgs& a, int c) { return (double)(c + a.L.ng + 1); }
 
-// get_heights_pass1 for one direction; grid = interior cells
-__global__ void k_heights_pass1(const StArgs a, int d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+// one of three values by a run-time direction (an indexed parameter array
+// would be copied to local memory by every thread)
+template <typename T>
+__device__ inline T by_dir(int d, T x, T y, T z) {
+    return d == 0 ? x : (d == 1 ? y : z);
+}
+
+// get_heights_pass1 for the three directions; grid = interior cells.  A pure
+// cell whose neighbour in the search direction is an interior cell of its own
+// phase abandons the search there (its s = 1), so the flags of the cell and its
+// six neighbours decide for all but the cells beside an interface or at the
+// edge of the domain: one byte a cell where every cell read its fraction and
+// flag in three passes (128^3: 130 to 9 us for the pass).
+__global__ void k_heights_pass1(const StArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
     if (i >= a.L.n[0]) return;
-    long n = lidx(a.L, i, j, k);
-    int f = a.f[n];
+    const long n = lidx(a.L, i, j, k);
+    const int f = a.f[n];
     if (f / 2 != 0) return;
-    for (int sign = -1; sign <= 1; sign += 2) {
-        int c[3] = {i, j, k};
+    const int nx = a.L.n[0], ny = a.L.n[1], nz = a.L.n[2];
+    const long sy = a.L.pitch, sz = a.L.plane;
+    const int fw = a.f[n - 1], fe = a.f[n + 1], fs = a.f[n - sy], fn = a.f[n + sy], fb = a.f[n - sz], ft = a.f[n + sz];
+    const bool inner = i > 0 && i < nx - 1 && j > 0 && j < ny - 1 && k > 0 && k < nz - 1;
+    if (inner && fw == f && fe == f && fs == f && fn == f && fb == f && ft == f) return;
+#pragma unroll 1
+    for (int q = 0; q < 6; q++) {
+        const int d = q >> 1, sign = q & 1 ? 1 : -1;
+        const int nd = by_dir(d, nx, ny, nz), edge = sign < 0 ? 0 : nd - 1;
+        const int f1 = sign < 0 ? by_dir(d, fw, fs, fb) : by_dir(d, fe, fn, ft);
+        int cd = by_dir(d, i, j, k);
+        if (f1 == f && cd != edge) continue;
+        const long st = by_dir(d, 1L, sy, sz) * sign;
         int normalsign = (2 * f - 1) * sign;
         int index = 2 * d + 1 + (-normalsign + 1) / 2;
         double* H = Hidx(a, index);
         int other = 1 - f;
-        int climitp1 = (sign < 0 ? 0 : a.L.n[d] - 1) + sign;
+        int climitp1 = edge + sign;
         double hp = 0.0;
-        int s = 0, c0 = c[d], c1 = c0 + sign * kNdepth;
+        int s = 0, c0 = cd, c1 = c0 + sign * kNdepth;
+        long cc = n;
         while (true) {
-            long cc = at(a, c);
             int fc = a.f[cc];
             bool same = s > 0 && fc == f;
             hp = hp + (a.c[cc] - 0.5) * normalsign;
-            bool abandon = same || fc == other || c[d] == climitp1 || s == 2 * kNdepth;
+            bool abandon = same || fc == other || cd == climitp1 || s == 2 * kNdepth;
             if (!abandon) {
                 s++;
-                c[d] += sign;
+                cd += sign;
+                cc += st;
                 continue;
             }
             if (fc == other) {
                 // full height; a downward search leaves interior stacks to their lower end
-                if (sign < 0 && c[d] != climitp1) break;
+                if (sign < 0 && cd != climitp1) break;
                 hp = hp + (2 * kNdepth - s) * (a.c[cc] - 0.5) * normalsign;
-                while (c[d] != c0 - sign) {
-                    H[at(a, c)] = hp + fidx(a, c1) - fidx(a, c[d]);
-                    c[d] -= sign;
+                while (cd != c0 - sign) {
+                    // above kHalfBig it would be reset to "not computed" (at the
+                    // domain's edge by pass 2, which takes it for a partial height)
+                    const double h = hp + fidx(a, c1) - fidx(a, cd);
+                    H[cc] = h > kHalfBig && cd != 0 && cd != nd - 1 ? kUncomputed : h;
+                    cd -= sign;
+                    cc -= st;
                 }
-            } else if (c[d] == climitp1) {
+            } else if (cd == climitp1) {
                 hp = hp + (-a.c[cc] + 0.5) * normalsign;
-                c[d] -= sign;
-                H[at(a, c)] = hp + (double)(kBigint * s);
+                H[cc - st] = hp + (double)(kBigint * s);
             }
             break;
         }
     }
 }
 
-// get_heights_pass2 for one direction; one thread per column (l, m)
-__global__ void k_heights_pass2(const StArgs a, int d, int t2, int t3) {
-    int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-    if (l >= a.L.n[t2] || m >= a.L.n[t3]) return;
-    int c[3];
-    c[t2] = l; c[t3] = m;
+// get_heights_pass2, one thread per column and direction (blockIdx.z = d),
+// with the reset of what is left of the partial heights ("not computed"): they
+// lie in the first and last cell of a column only.  The cells beyond the
+// column's ends are its other end as pass 1 left it where d is periodic, so no
+// exchange of ghosts comes between the passes.
+__global__ void k_heights_pass2(const StArgs a, const Bnd B) {
+    const int d = blockIdx.z, nx = a.L.n[0], ny = a.L.n[1], nz = a.L.n[2];
+    const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+    if (l >= (d == 0 ? ny : nx) || m >= (d == 2 ? ny : nz)) return;
+    const int nd = by_dir(d, nx, ny, nz);
+    const long st = by_dir(d, 1L, a.L.pitch, a.L.plane);
+    const long n0 = d == 0 ? lidx(a.L, 0, l, m) : (d == 1 ? lidx(a.L, l, 0, m) : lidx(a.L, l, m, 0));
+    double g[2][2];   // the cells beyond the low and high end, of the two heights
+    for (int q = 0; q < 2; q++) {
+        const double* H = Hidx(a, 2 * d + 1 + q);
+        const bool per = by_dir(d, B.per[0], B.per[1], B.per[2]) != 0;
+        g[q][0] = H[per ? n0 + (long)(nd - 1) * st : n0 - st];
+        g[q][1] = H[per ? n0 : n0 + (long)nd * st];
+    }
     for (int sign = -1; sign <= 1; sign += 2)
-        for (int index = 2 * d + 1; index <= 2 * d + 2; index++) {
-            double* H = Hidx(a, index);
-            int cb = sign < 0 ? 0 : a.L.n[d] - 1;
-            c[d] = cb;
-            double hb = H[at(a, c)];
+        for (int q = 0; q < 2; q++) {
+            double* H = Hidx(a, 2 * d + 1 + q);
+            int cb = sign < 0 ? 0 : nd - 1;
+            double hb = H[n0 + cb * st];
             if (!(hb > kHalfBig && hb < 1e6)) continue;
-            c[d] = cb + sign;
-            double ha = H[at(a, c)];
-            c[d] = cb;
+            double ha = g[q][sign < 0 ? 0 : 1];
             if (ha < kHalfBig) {
-                H[at(a, c)] = ha + sign;
+                H[n0 + cb * st] = ha + sign;
             } else if (ha > kHalfBig && ha < 1e6) {
                 int sbelow = (int)floorf(__fdiv_rn((float)(hb + kHalfBig), (float)kBigint));
                 hb = hb - kBigint * sbelow;
@@ -113,24 +146,39 @@ __global__ void k_heights_pass2(const StArgs a, int d, int t2, int t3) {
                 if (sabove + sbelow - 1 <= 2 * kNdepth + 1) {
                     int c0 = cb - (sbelow - 1) * sign;
                     double cmiddle = fidx(a, c0) + sign * (sabove + sbelow - 1) * 0.5;
-                    c[d] = cb + 2 * sign;
-                    while (c[d] != c0 - sign) {
-                        H[at(a, c)] = ha + hb + cmiddle - fidx(a, c[d]);
-                        c[d] -= sign;
+                    // (the two cells beyond the end get theirs from the exchange that follows)
+                    for (int c = cb; c != c0 - sign; c -= sign) {
+                        const double h = ha + hb + cmiddle - fidx(a, c);
+                        H[n0 + c * st] = h > kHalfBig && c != 0 && c != nd - 1 ? kUncomputed : h;
                     }
                 }
             }
         }
+    for (int q = 0; q < 2; q++) {
+        double* H = Hidx(a, 2 * d + 1 + q);
+        for (int c = 0; c < nd; c += nd - 1)
+            if (H[n0 + c * st] > kHalfBig) H[n0 + c * st] = kUncomputed;
+    }
 }
 
-__global__ void k_heights_reset(double* __restrict__ H, long total) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t < total && H[t] > kHalfBig) H[t] = 2e6;
+// do_all_ghost (periodic images) of n fields, one behind the other
+__global__ void k_ghost_fields(double* __restrict__ f, long total, const Layout L, const Bnd B) {
+    int i, j, k;
+    if (!ghost_cell(L, blockIdx.x * (long)blockDim.x + threadIdx.x, i, j, k)) return;
+    int si = i, sj = j, sk = k;
+    if (B.per[0]) { if (si < 0) si += L.n[0]; else if (si >= L.n[0]) si -= L.n[0]; }
+    if (B.per[1]) { if (sj < 0) sj += L.n[1]; else if (sj >= L.n[1]) sj -= L.n[1]; }
+    if (B.per[2]) { if (sk < 0) sk += L.n[2]; else if (sk >= L.n[2]) sk -= L.n[2]; }
+    if (si == i && sj == j && sk == k) return;
+    double* const h = f + (long)blockIdx.y * total;
+    h[lidx(L, i, j, k)] = h[lidx(L, si, sj, sk)];
 }
 
 __global__ void k_fill_d(double* __restrict__ f, double v, long n) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t < n) f[t] = v;
+    const long n2 = n >> 1;
+    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n2; t += (long)gridDim.x * blockDim.x)
+        reinterpret_cast<double2*>(f)[t] = make_double2(v, v);
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) f[n - 1] = v;
 }
 
 static StArgs st_args(paris_ctx* c) {
@@ -147,19 +195,12 @@ static int heights(paris_ctx* c) {
     PARIS_CHECK(ctx_alloc_field(c, PARIS_FIELD_HEIGHT));
     const Layout& L = c->L;
     StArgs a = st_args(c);
-    PARIS_LAUNCH(c, k_fill_d, div_up(6 * L.total, 256), 256, 0, c->height, 2e6, 6 * L.total);
-    dim3 g(div_up(L.n[0], 128), L.n[1], L.n[2]);
-    for (int d = 0; d < 3; d++) PARIS_LAUNCH_N(c, "heights_pass1", c->N, k_heights_pass1, g, 128, 0, a, d);
-    for (int q = 0; q < 6; q++) PARIS_CHECK(ctx_ghost_fill(c, c->height + q * L.total));
-    for (int d = 0; d < 3; d++) {
-        int t2 = (d + 1) % 3, t3 = (d + 2) % 3;
-        if (t2 > t3) { int t = t2; t2 = t3; t3 = t; }
-        PARIS_LAUNCH_N(c, "heights_pass2", (long)L.n[t2] * L.n[t3], k_heights_pass2,
-                       dim3(div_up(L.n[t2], 128), L.n[t3]), 128, 0, a, d, t2, t3);
-        PARIS_LAUNCH(c, k_heights_reset, div_up(2 * L.total, 256), 256, 0, c->height + 2 * d * L.total,
-                     2 * L.total);
-    }
-    for (int q = 0; q < 6; q++) PARIS_CHECK(ctx_ghost_fill(c, c->height + q * L.total));
+    PARIS_LAUNCH(c, k_fill_d, (unsigned)(c->nsm * 8), 256, 0, c->height, kUncomputed, 6 * L.total);
+    PARIS_LAUNCH_N(c, "heights_pass1", 3 * c->N, k_heights_pass1, dim3(div_up(L.n[0], 128), L.n[1], L.n[2]), 128, 0, a);
+    const int nx = L.n[0], ny = L.n[1], nz = L.n[2], w = nx > ny ? nx : ny, h = ny > nz ? ny : nz;
+    PARIS_LAUNCH_N(c, "heights_pass2", (long)nx * ny + (long)ny * nz + (long)nx * nz, k_heights_pass2,
+                   dim3(div_up(w, 128), h, 3), 128, 0, a, c->bnd);
+    PARIS_LAUNCH(c, k_ghost_fields, dim3(div_up(ghost_count(L), 256), 6), 256, 0, c->height, L.total, L, c->bnd);
     return PARIS_OK;
 }
 
@@ -351,25 +392,42 @@ __device__ double curv_pass2(const CurvArgs& A, long n, int& nfound_out) {
     return kappa;
 }
 
-// interior mixed cells (flag 2), warp-aggregated append
-__global__ void k_mixed_interior(const int8_t* __restrict__ f, const Layout L, int* list, int* count) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-    long n = i < L.n[0] ? lidx(L, i, j, k) : 0;
-    bool mixed = i < L.n[0] && f[n] == 2;
-    unsigned m = __ballot_sync(0xffffffffu, mixed);
+// One pass over the ghosted arrays (blocks of a row, i - ng first): curvature
+// and kappaflag "not computed" (a pure interior cell will stay so), and the
+// interior mixed cells (flag 2) in a list, with one atomic per warp.
+__global__ void k_curv_init(double* __restrict__ kap, int8_t* __restrict__ kf, const int8_t* __restrict__ f,
+                            const Layout L, int* list, int* count) {
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) - L.ng, j = (int)blockIdx.y - L.ng,
+              k = (int)blockIdx.z - L.ng;
+    const bool in = i < L.n[0] + L.ng;
+    const long n = in ? lidx(L, i, j, k) : 0;
+    const bool inner = i >= 0 && i < L.n[0] && j >= 0 && j < L.n[1] && k >= 0 && k < L.n[2];
+    const bool mixed = inner && f[n] == 2;
+    if (in) {
+        kap[n] = kUncomputed;
+        kf[n] = inner && !mixed ? kUncomputable : kUndecided;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, mixed);
     if (!m) return;
-    int lane = threadIdx.x & 31, leader = __ffs(m) - 1, base = 0;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    int base = 0;
     if (lane == leader) base = atomicAdd(count, __popc(m));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (mixed) list[base + __popc(m & ((1u << lane) - 1u))] = (int)n;
 }
 
-__global__ void k_curv_init(double* __restrict__ kap, int8_t* __restrict__ kf, const int8_t* __restrict__ f,
-                            const Layout L, long total) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    kap[t] = kUncomputed;
-    kf[t] = kUndecided;
+// do_all_ghost of the curvature and its flag
+__global__ void k_curv_ghosts(double* __restrict__ kap, int8_t* __restrict__ kf, const Layout L, const Bnd B) {
+    int i, j, k;
+    if (!ghost_cell(L, blockIdx.x * (long)blockDim.x + threadIdx.x, i, j, k)) return;
+    int si = i, sj = j, sk = k;
+    if (B.per[0]) { if (si < 0) si += L.n[0]; else if (si >= L.n[0]) si -= L.n[0]; }
+    if (B.per[1]) { if (sj < 0) sj += L.n[1]; else if (sj >= L.n[1]) sj -= L.n[1]; }
+    if (B.per[2]) { if (sk < 0) sk += L.n[2]; else if (sk >= L.n[2]) sk -= L.n[2]; }
+    if (si == i && sj == j && sk == k) return;
+    const long n = lidx(L, i, j, k), m = lidx(L, si, sj, sk);
+    kap[n] = kap[m];
+    kf[n] = kf[m];
 }
 
 __global__ void __launch_bounds__(128) k_curv_pass1(const CurvArgs A) {
@@ -410,28 +468,18 @@ __global__ void __launch_bounds__(128) k_curv_pass2(const CurvArgs A) {
     int cnt = *A.count;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += gridDim.x * blockDim.x) {
         long n = A.list[q];
-        if (A.kf[n] <= 2) continue;
-        int nf;
-        double kap = curv_pass2(A, n, nf);
-        if (nf > 0) A.kf[n] = kUncomputable;
-        else { A.kap[n] = kap; A.kf[n] = 3; }
+        double kap = A.kap[n];
+        if (A.kf[n] > 2) {
+            int nf;
+            const double fit = curv_pass2(A, n, nf);
+            A.kf[n] = nf > 0 ? kUncomputable : 3;
+            if (nf > 0) continue;
+            kap = fit;
+        }
+        // clipped, as every computed curvature (its images are exchanged afterwards)
+        if (fabs(kap) > kKappaMax) kap = copysign(1.0, kap) * kKappaMax;
+        A.kap[n] = kap;
     }
-}
-
-// pure interior cells are UNCOMPUTABLE
-__global__ void k_curv_pure(const int8_t* __restrict__ f, int8_t* __restrict__ kf, const Layout L) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-    if (i >= L.n[0]) return;
-    long n = lidx(L, i, j, k);
-    if (f[n] != 2) kf[n] = kUncomputable;
-}
-
-__global__ void k_curv_clip(double* __restrict__ kap, const int8_t* __restrict__ kf, long total) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= total || kf[t] >= kUncomputable) return;
-    double k = kap[t];
-    if (fabs(k) > kKappaMax) k = copysign(1.0, k) * kKappaMax;
-    kap[t] = k;
 }
 
 static int curvatures(paris_ctx* c) {
@@ -451,20 +499,15 @@ static int curvatures(paris_ctx* c) {
     A.do_rotation = c->d.do_rotation;
     A.use_full_heights = c->d.use_full_heights;
     A.epsc = c->d.epsc;
-    dim3 g(div_up(L.n[0], 128), L.n[1], L.n[2]);
     PARIS_CUDA_TRY(c, cudaMemsetAsync(c->st_count, 0, sizeof(int), c->stream));
-    PARIS_LAUNCH(c, k_mixed_interior, g, 128, 0, c->flag, L, c->st_list, c->st_count);
-    PARIS_LAUNCH(c, k_curv_init, div_up(L.total, 256), 256, 0, A.kap, A.kf, c->flag, L, L.total);
-    unsigned gg = c->nsm * 8;
+    PARIS_LAUNCH(c, k_curv_init, dim3(div_up(L.n[0] + 2 * L.ng, 128), L.n[1] + 2 * L.ng, L.n[2] + 2 * L.ng), 128, 0,
+                 A.kap, A.kf, c->flag, L, c->st_list, c->st_count);
+    const unsigned gg = c->nsm * 8, G = div_up(ghost_count(L), 256);
     PARIS_LAUNCH_N(c, "curvature_pass1", 0L, k_curv_pass1, gg, 128, 0, A);
-    PARIS_CHECK(ctx_ghost_fill(c, A.kap));
-    PARIS_CHECK(ctx_ghost_fill_i8(c, A.kf));
+    PARIS_LAUNCH(c, k_curv_ghosts, G, 256, 0, A.kap, A.kf, L, c->bnd);
     PARIS_LAUNCH(c, k_curv_average, gg, 128, 0, A);
     PARIS_LAUNCH_N(c, "curvature_pass2", 0L, k_curv_pass2, gg, 128, 0, A);
-    PARIS_LAUNCH(c, k_curv_pure, g, 128, 0, c->flag, A.kf, L);
-    PARIS_CHECK(ctx_ghost_fill(c, A.kap));
-    PARIS_CHECK(ctx_ghost_fill_i8(c, A.kf));
-    PARIS_LAUNCH(c, k_curv_clip, div_up(L.total, 256), 256, 0, A.kap, A.kf, L.total);
+    PARIS_LAUNCH(c, k_curv_ghosts, G, 256, 0, A.kap, A.kf, L, c->bnd);
     return PARIS_OK;
 }
 
