@@ -8,6 +8,8 @@
 // partials added in block order by one block per column.  The max is
 // order-independent, so the time step equals the reference's bit for bit;
 // the sums differ from its k,j,i loop order only by rounding.
+#include <cmath>
+
 #include "ctx.cuh"
 #include "plic.cuh"
 
@@ -38,6 +40,7 @@ struct StatsArgs {
     double top_layer;                                   // xLength*zLength*(yLength-height4Stats)
     int force, bubble, phase_inv, turb;
     int per[3];
+    double r2x, r2y, r2z;                               // exact 1 / (x(i+1) - x(i-1)) etc. (EXACT)
 };
 
 // PLIC interface area of a mixed cell (mycs normal + AREA3D,
@@ -57,8 +60,14 @@ __device__ __noinline__ double cell_area(const double* __restrict__ c, long n, c
     return 0.0;
 }
 
-// calcStats main loop, paris.f90:1136-1239; s[q-1] is mystats(q)
-__global__ void __launch_bounds__(kThreads) k_calc_stats(const StatsArgs a, const Layout L, double* part) {
+// calcStats main loop, paris.f90:1136-1239; s[q-1] is mystats(q).  Bound by the
+// latency of its forty-odd neighbour loads: with two blocks per SM (some of the
+// 25 sums spill) 256x256x512 takes 2.01 ms, with one and no spills 3.64.  EXACT:
+// every x(i+1) - x(i-1) is the same power of two, likewise y and z, and the six
+// divisions of the vorticity are products by the exact reciprocals, the same
+// doubles (1.70 ms).
+template <bool EXACT>
+__global__ void __launch_bounds__(kThreads, 2) k_calc_stats(const StatsArgs a, const Layout L, double* part) {
     __shared__ double sh[32];
     double s[kNS];
 #pragma unroll
@@ -110,13 +119,15 @@ __global__ void __launch_bounds__(kThreads) k_calc_stats(const StatsArgs a, cons
             s[19] = s[19] + rn * a.gy * a.y[J] * vol * cc;
             s[20] = s[20] + rn * a.gy * a.y[J] * vol * (1.0 - cc);
         }
-        const double dyc = a.y[J + 1] - a.y[J - 1], dzc = a.z[K + 1] - a.z[K - 1], dxc = a.x[I + 1] - a.x[I - 1];
-        const double d1 = 0.5 * (a.w[n + nn] + a.w[n + nn + t] - a.w[n - nn] - a.w[n - nn + t]) / dyc -
-                          0.5 * (a.v[n + t] + a.v[n + nn + t] - a.v[n - t] - a.v[n + nn - t]) / dzc;
-        const double d2 = 0.5 * (a.u[n + t] + a.u[n + e + t] - a.u[n - t] - a.u[n + e - t]) / dzc -
-                          0.5 * (a.w[n + e] + a.w[n + e + t] - a.w[n - e] - a.w[n - e + t]) / dxc;
-        const double d3 = 0.5 * (a.v[n + e] + a.v[n + e + nn] - a.v[n - e] - a.v[n - e + nn]) / dxc -
-                          0.5 * (a.u[n + nn] + a.u[n + e + nn] - a.u[n - nn] - a.u[n + e - nn]) / dyc;
+        const double dyc = EXACT ? a.r2y : a.y[J + 1] - a.y[J - 1], dzc = EXACT ? a.r2z : a.z[K + 1] - a.z[K - 1],
+                     dxc = EXACT ? a.r2x : a.x[I + 1] - a.x[I - 1];
+        auto over = [](double q, double d) { return EXACT ? q * d : q / d; };
+        const double d1 = over(0.5 * (a.w[n + nn] + a.w[n + nn + t] - a.w[n - nn] - a.w[n - nn + t]), dyc) -
+                          over(0.5 * (a.v[n + t] + a.v[n + nn + t] - a.v[n - t] - a.v[n + nn - t]), dzc);
+        const double d2 = over(0.5 * (a.u[n + t] + a.u[n + e + t] - a.u[n - t] - a.u[n + e - t]), dzc) -
+                          over(0.5 * (a.w[n + e] + a.w[n + e + t] - a.w[n - e] - a.w[n - e + t]), dxc);
+        const double d3 = over(0.5 * (a.v[n + e] + a.v[n + e + nn] - a.v[n - e] - a.v[n - e + nn]), dxc) -
+                          over(0.5 * (a.u[n + nn] + a.u[n + e + nn] - a.u[n - nn] - a.u[n + e - nn]), dyc);
         const double ens = 0.5 * (d1 * d1 + d2 * d2 + d3 * d3);
         s[21] = s[21] + ens * vol * cc;
         s[22] = s[22] + ens * vol * (1.0 - cc);
@@ -141,6 +152,18 @@ __global__ void k_stats_finish(const double* __restrict__ part, double* out, int
     for (int b = threadIdx.x; b < nb; b += blockDim.x) v += part[(long)q * kRedBlocks + b];
     v = block_sum<kThreads>(v, sh);
     if (threadIdx.x == 0) out[q] = v;
+}
+
+// every x(i+1) - x(i-1) of the interior is the same power of two: *r its
+// reciprocal, exact
+bool uniform_pow2_span(const std::vector<double>& x, int n, int g, double* r) {
+    const double d = x[g + 1] - x[g - 1];
+    for (int i = g; i < n + g; i++)
+        if (x[i + 1] - x[i - 1] != d) return false;
+    int ex;
+    if (std::frexp(d, &ex) != 0.5) return false;
+    *r = 1.0 / d;
+    return true;
 }
 
 double min_dx(const paris_ctx* c) {
@@ -225,8 +248,11 @@ extern "C" int paris_calc_stats(paris_handle_t c, const paris_stats_opts* opts, 
     a.phase_inv = (o.test_flags & PARIS_STATS_PHASE_INVERSION) != 0;
     a.turb = (o.test_flags & PARIS_STATS_TURB) != 0;
     for (int q = 0; q < 3; q++) a.per[q] = c->bnd.per[q];
-    const unsigned nb = red_grid(c, k_calc_stats, kThreads);
-    PARIS_LAUNCH_N(c, "calc_stats", c->N, k_calc_stats, nb, kRowBlock, 0, a, c->L, c->stats_part);
+    const bool exact = uniform_pow2_span(c->h_x, d.nx, d.ng, &a.r2x) && uniform_pow2_span(c->h_y, d.ny, d.ng, &a.r2y) &&
+                       uniform_pow2_span(c->h_z, d.nz, d.ng, &a.r2z);
+    const unsigned nb = exact ? red_grid(c, k_calc_stats<true>, kThreads) : red_grid(c, k_calc_stats<false>, kThreads);
+    if (exact) PARIS_LAUNCH_N(c, "calc_stats", c->N, k_calc_stats<true>, nb, kRowBlock, 0, a, c->L, c->stats_part);
+    else PARIS_LAUNCH_N(c, "calc_stats", c->N, k_calc_stats<false>, nb, kRowBlock, 0, a, c->L, c->stats_part);
     PARIS_LAUNCH(c, k_stats_finish, kNS, kThreads, 0, c->stats_part, c->stats_out, (int)nb);
     double ms[kNS];
     PARIS_CUDA_TRY(c, cudaMemcpyAsync(ms, c->stats_out, sizeof ms, cudaMemcpyDeviceToHost, c->stream));
