@@ -68,13 +68,12 @@ __device__ inline double inter_q(const QuickCoef* __restrict__ c, double y0, dou
 // Both candidates of the upwind point are loaded before the upwind test, so
 // the four loads of a face value are independent (one memory round trip
 // instead of two); the arithmetic is unchanged.
-template <bool R>
 __device__ inline double quick_same(const double* __restrict__ phi, long n, long st, const QuickCoef* __restrict__ Q,
                                     int t) {
     const double pm2 = phi[n - 2 * st], pm1 = phi[n - st], p0 = phi[n], pp1 = phi[n + st];
     const bool up = pm1 + p0 > 0.0;
     const double y2 = up ? pm2 : pp1;
-    return inter_q<R>(Q + 4 * t + (up ? 0 : 1), up ? pm1 : p0, up ? p0 : pm1, y2);
+    return inter_q<false>(Q + 4 * t + (up ? 0 : 1), up ? pm1 : p0, up ? p0 : pm1, y2);
 }
 // the same with the two coefficient sets of a uniform axis
 __device__ inline QuickCoef pick(bool up, const QuickCoef& a, const QuickCoef& b) {
@@ -105,13 +104,12 @@ __device__ inline double quick_same_u(const double* __restrict__ phi, long n, lo
 
 // QUICK value of a component on the face jj+1/2 of another axis, upwinded
 // by vel(n) + vel(n + sc)
-template <bool R>
 __device__ inline double quick_cross(const double* __restrict__ phi, const double* __restrict__ vel, long n, long st,
                                      long sc, const QuickCoef* __restrict__ Q, int t) {
     const double v0 = vel[n], v1 = vel[n + sc];
     const double am = phi[n - st], a = phi[n], b = phi[n + st], bp = phi[n + 2 * st];
     const bool up = v0 + v1 > 0.0;
-    return inter_q<R>(Q + 4 * t + (up ? 2 : 3), up ? a : b, up ? b : a, up ? am : bp);
+    return inter_q<false>(Q + 4 * t + (up ? 2 : 3), up ? a : b, up ? b : a, up ? am : bp);
 }
 template <bool C>
 __device__ inline double quick_cross_u(const double* __restrict__ phi, const double* __restrict__ vel, long n, long st,
@@ -123,12 +121,6 @@ __device__ inline double quick_cross_u(const double* __restrict__ phi, const dou
     return inter_u<C>(c, up ? a : b, up ? b : a, up ? am : bp);
 }
 
-// x / den, or x * (1/den) where that reciprocal is exact (same double)
-template <bool R>
-__device__ inline double over(double x, double den, double rden) {
-    return R ? x * rden : x / den;
-}
-
 // The coefficients of a uniform grid: every index carries the same four
 // coefficient sets and metric reciprocals per axis (checked bit for bit on
 // the host), passed by value so the kernel loads no table.
@@ -138,41 +130,103 @@ struct QuickUniform {
 };
 
 // momentumConvectionQUICK: du, dv, dw assigned on the faces project_velocity
-// updates (is..ieu etc.)
-template <bool R>
-__global__ void __launch_bounds__(256) k_conv_quick(Vel V, double* __restrict__ du, double* __restrict__ dv,
+// updates (is..ieu etc.), with the divisions of inter().
+//
+// A face value costs some 150 instructions here (four divisions), so values are shared
+// where that is free: a thread marches up a column and carries the values of
+// the z faces, a warp holds 30 columns of a row and one on either side and
+// hands the values of the x faces on by shuffle; the y faces are formed twice:
+// twelve face values per cell instead of eighteen.  An outer lane forms only
+// what its neighbour takes, at cells within the ghost layers' stencil reach.
+// The coefficients of the x axis, different in every lane, stay in registers
+// (as table rows of 160 bytes they took a sector per lane in every face value).
+// Warps in flight count for more than registers: eight blocks of 128 per SM (64
+// registers, some spilled) 425 us at 200x168x121, 479 with six, 529 with four,
+// 604 with a thread per cell and eighteen face values.
+// The uniform forms below, with a third of the operations, are slower this way
+// (256x256x512: 1.01 ms against 0.88).
+__global__ void __launch_bounds__(128, 8) k_conv_quick(Vel V, double* __restrict__ du, double* __restrict__ dv,
                                                     double* __restrict__ dw, const Layout L, const Bnd B, const Geo G,
-                                                    const MomTab T) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= L.n[0] || j >= L.n[1] || k >= L.n[2]) return;
-    const int g = L.ng;
-    const long n = lidx(L, i, j, k), sx = 1, sy = L.pitch, sz = L.plane;
+                                                    const MomTab T, int zc) {
+    const int n0 = L.n[0], n1 = L.n[1], n2 = L.n[2], g = L.ng;
+    const int lane = threadIdx.x, i = (int)(blockIdx.x * 30) + lane - 1, j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (j >= n1) return;   // the whole warp
+    const int k0 = blockIdx.z * zc, k1 = min(k0 + zc, n2);
+    const bool in = i >= 0 && i < n0, left = i >= -1 && i < n0, right = i >= 0 && i <= n0;
+    const bool out = in && lane >= 1 && lane <= 30;
+    const long sx = 1, sy = L.pitch, sz = L.plane;
     const double *u = V.u, *v = V.v, *w = V.w;
-    const QuickCoef *QX = T.q[0], *QY = T.q[1], *QZ = T.q[2];
-    const int I = i + g, J = j + g, K = k + g;
-    if (i < L.n[0] - 1 || B.per[0]) {
-        double a = quick_same<R>(u, n + sx, sx, QX, I + 1), b = quick_same<R>(u, n, sx, QX, I);
-        double w2 = quick_cross<R>(u, v, n, sy, sx, QY, J), w2m = quick_cross<R>(u, v, n - sy, sy, sx, QY, J - 1);
-        double w3 = quick_cross<R>(u, w, n, sz, sx, QZ, K), w3m = quick_cross<R>(u, w, n - sz, sz, sx, QZ, K - 1);
-        du[n] = over<R>(-(a * a - b * b), G.a[0].dh[I], T.rdh[0][I])
-            - over<R>(0.5 * ((v[n] + v[n + sx]) * w2 - (v[n - sy] + v[n + sx - sy]) * w2m), G.a[1].d[J], T.rd[1][J])
-            - over<R>(0.5 * ((w[n] + w[n + sx]) * w3 - (w[n - sz] + w[n + sx - sz]) * w3m), G.a[2].d[K], T.rd[2][K]);
+    const int I = i + g, J = j + g;
+    QuickCoef qx[4] = {};   // the x axis at I
+    if (left || right)
+        for (int s = 0; s < 4; s++) {
+            qx[s].xi = T.q[0][4 * I + s].xi;
+            qx[s].k = T.q[0][4 * I + s].k;
+        }
+    const double ddx = in ? G.a[0].d[I] : 1.0, ddxh = in ? G.a[0].dh[I] : 1.0;
+    // the value of phi at its own cell centre along axis a, table index t
+    auto same = [&](const double* phi, long n, int a, int t) {
+        const long st = a == 0 ? sx : (a == 1 ? sy : sz);
+        if (a != 0) return quick_same(phi, n, st, T.q[a], t);
+        const double pm2 = phi[n - 2 * st], pm1 = phi[n - st], p0 = phi[n], pp1 = phi[n + st];
+        const bool up = pm1 + p0 > 0.0;
+        const QuickCoef c = pick(up, qx[0], qx[1]);
+        return inter_q<false>(&c, up ? pm1 : p0, up ? p0 : pm1, up ? pm2 : pp1);
+    };
+    // the value of phi on the face + 1/2 of axis a, upwinded by vel(n) + vel(n + sc)
+    auto cross = [&](const double* phi, const double* vel, long n, int a, long sc, int t) {
+        const long st = a == 0 ? sx : (a == 1 ? sy : sz);
+        if (a != 0) return quick_cross(phi, vel, n, st, sc, T.q[a], t);
+        const double v0 = vel[n], v1 = vel[n + sc];
+        const double am = phi[n - st], p = phi[n], b = phi[n + st], bp = phi[n + 2 * st];
+        const bool up = v0 + v1 > 0.0;
+        const QuickCoef c = pick(up, qx[2], qx[3]);
+        return inter_q<false>(&c, up ? p : b, up ? b : p, up ? am : bp);
+    };
+    auto by_d = [&](double x, int a, int t) { return x / (a == 0 ? ddx : G.a[a].d[t]); };
+    auto by_dh = [&](double x, int a, int t) { return x / (a == 0 ? ddxh : G.a[a].dh[t]); };
+    long n = lidx(L, i, j, k0);
+    double uz = 0.0, vz = 0.0, sw = 0.0;   // z fluxes of u and v through the face below, w at the centre
+    if (in) {
+        const long m = n - sz;
+        uz = (w[m] + w[m + sx]) * cross(u, w, m, 2, sx, k0 + g - 1);
+        vz = (w[m] + w[m + sy]) * cross(v, w, m, 2, sy, k0 + g - 1);
+        sw = same(w, n, 2, k0 + g);
     }
-    if (j < L.n[1] - 1 || B.per[1]) {
-        double a = quick_same<R>(v, n + sy, sy, QY, J + 1), b = quick_same<R>(v, n, sy, QY, J);
-        double w1 = quick_cross<R>(v, u, n, sx, sy, QX, I), w1m = quick_cross<R>(v, u, n - sx, sx, sy, QX, I - 1);
-        double w3 = quick_cross<R>(v, w, n, sz, sy, QZ, K), w3m = quick_cross<R>(v, w, n - sz, sz, sy, QZ, K - 1);
-        dv[n] = over<R>(-0.5 * ((u[n] + u[n + sy]) * w1 - (u[n - sx] + u[n - sx + sy]) * w1m), G.a[0].d[I], T.rd[0][I])
-            - over<R>(a * a - b * b, G.a[1].dh[J], T.rdh[1][J])
-            - over<R>(0.5 * ((w[n] + w[n + sy]) * w3 - (w[n - sz] + w[n + sy - sz]) * w3m), G.a[2].d[K], T.rd[2][K]);
-    }
-    if (k < L.n[2] - 1 || B.per[2]) {
-        double a = quick_same<R>(w, n + sz, sz, QZ, K + 1), b = quick_same<R>(w, n, sz, QZ, K);
-        double w1 = quick_cross<R>(w, u, n, sx, sz, QX, I), w1m = quick_cross<R>(w, u, n - sx, sx, sz, QX, I - 1);
-        double w2 = quick_cross<R>(w, v, n, sy, sz, QY, J), w2m = quick_cross<R>(w, v, n - sy, sy, sz, QY, J - 1);
-        dw[n] = over<R>(-0.5 * ((u[n] + u[n + sz]) * w1 - (u[n - sx] + u[n - sx + sz]) * w1m), G.a[0].d[I], T.rd[0][I])
-            - over<R>(0.5 * ((v[n] + v[n + sz]) * w2 - (v[n - sy] + v[n - sy + sz]) * w2m), G.a[1].d[J], T.rd[1][J])
-            - over<R>(a * a - b * b, G.a[2].dh[K], T.rdh[2][K]);
+    for (int k = k0; k < k1; k++, n += sz) {
+        const int K = k + g;
+        double su = 0.0, vx = 0.0, wx = 0.0;   // u at the centre, x fluxes of v and w through the face i+1/2
+        if (right) su = same(u, n, 0, I);
+        if (left) {
+            vx = (u[n] + u[n + sy]) * cross(v, u, n, 0, sy, I);
+            wx = (u[n] + u[n + sz]) * cross(w, u, n, 0, sz, I);
+        }
+        const double sue = __shfl_down_sync(0xffffffffu, su, 1);
+        const double vxw = __shfl_up_sync(0xffffffffu, vx, 1), wxw = __shfl_up_sync(0xffffffffu, wx, 1);
+        if (out) {
+            const double uzt = (w[n] + w[n + sx]) * cross(u, w, n, 2, sx, K);
+            const double vzt = (w[n] + w[n + sy]) * cross(v, w, n, 2, sy, K);
+            const double swt = same(w, n + sz, 2, K + 1);
+            if (i < n0 - 1 || B.per[0]) {
+                const double w2 = cross(u, v, n, 1, sx, J), w2m = cross(u, v, n - sy, 1, sx, J - 1);
+                du[n] = by_dh(-(sue * sue - su * su), 0, I) -
+                        by_d(0.5 * ((v[n] + v[n + sx]) * w2 - (v[n - sy] + v[n + sx - sy]) * w2m), 1, J) -
+                        by_d(0.5 * (uzt - uz), 2, K);
+            }
+            if (j < n1 - 1 || B.per[1]) {
+                const double a = same(v, n + sy, 1, J + 1), b = same(v, n, 1, J);
+                dv[n] = by_d(-0.5 * (vx - vxw), 0, I) - by_dh(a * a - b * b, 1, J) - by_d(0.5 * (vzt - vz), 2, K);
+            }
+            if (k < n2 - 1 || B.per[2]) {
+                const double w2 = cross(w, v, n, 1, sz, J), w2m = cross(w, v, n - sy, 1, sz, J - 1);
+                dw[n] = by_d(-0.5 * (wx - wxw), 0, I) -
+                        by_d(0.5 * ((v[n] + v[n + sz]) * w2 - (v[n - sy] + v[n - sy + sz]) * w2m), 1, J) -
+                        by_dh(swt * swt - sw * sw, 2, K);
+            }
+            uz = uzt;
+            vz = vzt;
+            sw = swt;
+        }
     }
 }
 
@@ -268,9 +322,13 @@ __global__ void k_conv_onedim(Vel V, double* __restrict__ du, double* __restrict
 
 namespace {
 
-// explicitMomDiff, paris.f90:2757-2808 (adds to du, dv, dw)
+// explicitMomDiff, paris.f90:2757-2808 (adds to du, dv, dw).  Bound by the
+// latency of its loads: more warps per SM pay, at 32 registers on a uniform grid
+// (256x256x512: 1.02 to 0.93 ms) and 40 with the metric tables (200x168x121: 213
+// to 178 us); all loads of a cell up front, at half the warps, took 2.01 ms and
+// 293 us.
 template <bool UNI>
-__global__ void __launch_bounds__(256) k_mom_diff(Vel V, const double* __restrict__ rho, const double* __restrict__ mu,
+__global__ void __launch_bounds__(256, UNI ? 8 : 6) k_mom_diff(Vel V, const double* __restrict__ rho, const double* __restrict__ mu,
                                                   double* __restrict__ du, double* __restrict__ dv,
                                                   double* __restrict__ dw, const Layout L, const Bnd B, const MomTab T,
                                                   const QuickUniform Q) {
@@ -548,20 +606,22 @@ extern "C" int paris_momentum_convection(paris_handle_t c, int32_t scheme) {
         bool canon = uniform;   // every coefficient set xi = 1/2, k = -1 exactly
         for (int a = 0; a < 3 && canon; a++)
             for (int v = 0; v < 4; v++) canon = canon && U.q[a][v].xi == 0.5 && U.q[a][v].k == -1.0;
-        if (canon)
-            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick_uniform<true>, cgrid(c->L), cblock(), 0, vel(c),
-                           c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV], c->fld[PARIS_FIELD_DW], c->L, c->bnd, U);
-        else if (uniform)
-            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick_uniform<false>, cgrid(c->L), cblock(), 0, vel(c),
-                           c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV], c->fld[PARIS_FIELD_DW], c->L, c->bnd, U);
-        else if (exact)
-            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick<true>, cgrid(c->L), cblock(), 0, vel(c),
-                           c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV], c->fld[PARIS_FIELD_DW], c->L, c->bnd, geo(c),
-                           T);
-        else
-            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick<false>, cgrid(c->L), cblock(), 0, vel(c),
-                           c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV], c->fld[PARIS_FIELD_DW], c->L, c->bnd, geo(c),
-                           T);
+        double *du = c->fld[PARIS_FIELD_DU], *dv = c->fld[PARIS_FIELD_DV], *dw = c->fld[PARIS_FIELD_DW];
+        if (canon) {
+            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick_uniform<true>, cgrid(c->L), cblock(), 0, vel(c), du, dv,
+                           dw, c->L, c->bnd, U);
+        } else if (uniform) {
+            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick_uniform<false>, cgrid(c->L), cblock(), 0, vel(c), du,
+                           dv, dw, c->L, c->bnd, U);
+        } else {
+            // columns of up to 16 planes, fewer where that leaves SMs without blocks
+            const long tiles = (long)div_up(c->L.n[0], 30) * div_up(c->L.n[1], 4);
+            int zc = 16;
+            while (zc > 4 && tiles * div_up(c->L.n[2], zc) < 8L * c->nsm) zc /= 2;
+            PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_quick,
+                           dim3(div_up(c->L.n[0], 30), div_up(c->L.n[1], 4), div_up(c->L.n[2], zc)), dim3(32, 4), 0,
+                           vel(c), du, dv, dw, c->L, c->bnd, geo(c), T, zc);
+        }
     } else
         PARIS_LAUNCH_N(c, "mom_convection", c->N, k_conv_onedim, cgrid(c->L), cblock(), 0, vel(c),
                        c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV], c->fld[PARIS_FIELD_DW], c->L, c->bnd, geo(c),
