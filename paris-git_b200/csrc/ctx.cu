@@ -63,8 +63,11 @@ int ctx_alloc_field(paris_ctx* c, int field) {
 }
 
 // ---- ghost fills ----------------------------------------------------------
+// up to three arrays per launch (blockIdx.y): a face's few thousand copies
+// take less time than a launch
 template <typename T>
-__global__ void k_ghost_fill(T* __restrict__ f, const Layout L, const Bnd B) {
+__global__ void k_ghost_fill(T* f0, T* f1, T* f2, const Layout L, const Bnd B) {
+    T* const __restrict__ f = blockIdx.y == 0 ? f0 : (blockIdx.y == 1 ? f1 : f2);
     long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
     int i, j, k;
     if (!ghost_cell(L, t, i, j, k)) return;
@@ -76,15 +79,16 @@ __global__ void k_ghost_fill(T* __restrict__ f, const Layout L, const Bnd B) {
     f[lidx(L, i, j, k)] = f[lidx(L, si, sj, sk)];
 }
 
-int ctx_ghost_fill(paris_ctx* c, double* f) {
+int ctx_ghost_fill(paris_ctx* c, double* f0, double* f1, double* f2) {
     long G = ghost_count(c->L);
-    PARIS_LAUNCH(c, k_ghost_fill<double>, div_up(G, 256), 256, 0, f, c->L, c->bnd);
+    const unsigned nf = f2 ? 3 : (f1 ? 2 : 1);
+    PARIS_LAUNCH(c, k_ghost_fill<double>, dim3(div_up(G, 256), nf), 256, 0, f0, f1, f2, c->L, c->bnd);
     return PARIS_OK;
 }
 
 int ctx_ghost_fill_i8(paris_ctx* c, int8_t* f) {
     long G = ghost_count(c->L);
-    PARIS_LAUNCH(c, k_ghost_fill<int8_t>, div_up(G, 256), 256, 0, f, c->L, c->bnd);
+    PARIS_LAUNCH(c, k_ghost_fill<int8_t>, div_up(G, 256), 256, 0, f, (int8_t*)nullptr, (int8_t*)nullptr, c->L, c->bnd);
     return PARIS_OK;
 }
 

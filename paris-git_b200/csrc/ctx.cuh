@@ -144,7 +144,8 @@ unsigned red_grid(paris_ctx* c, K kernel, int threads) {
 
 // internal API (ctx.cu)
 int ctx_alloc_field(paris_ctx* c, int field);
-int ctx_ghost_fill(paris_ctx* c, double* f);         // do_all_ghost (periodic wrap)
+// do_all_ghost (periodic wrap) of one to three distinct arrays
+int ctx_ghost_fill(paris_ctx* c, double* f0, double* f1 = nullptr, double* f2 = nullptr);
 int ctx_ghost_fill_i8(paris_ctx* c, int8_t* f);
 int ctx_reduce_finish(paris_ctx* c, int nslots, double* out_host, int op_max = 0);
 int ctx_ensure_matrix(paris_ctx* c);
@@ -173,6 +174,7 @@ inline VofJet ctx_vof_jet(const paris_ctx* c) {
 // vof.cu: one split sweep (swpz or swpr, then SetVOFBC, get_flags_and_clip
 // and the ghosts) along d of the volume fraction src into dst with its flags;
 // us: the face velocity of the sweep, cg: c_mask for the Weymouth-Yue sweep
+int vof_sweep_list(paris_ctx* c, int d, const double* src);   // first: its mixed cells
 int vof_sweep_dir(paris_ctx* c, int d, double dt, const double* src, double* dst, int8_t* flag, const double* us,
                   const uint8_t* cg);
 // vof.cu: c_mask (vofmodules.f90:1295-1305) over total cells

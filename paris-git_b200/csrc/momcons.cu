@@ -17,9 +17,12 @@
 //      mixed (get_velocity_from_momentum_staggered :1486-1534 /
 //      get_velocity_from_momentum_centered :1451-1484), then the ghosts.
 //
-// One thread per cell throughout; the flux kernels cover the cells whose
-// fluxes reach the interior (the interior across d, one cell beyond it along
-// d), like the VOF sweeps.  Built with -fmad=false so that each expression
+// One thread per cell, except that the mixed cells (0 < c < 1), a few per cent
+// of a box but each a long chain of divisions and roots, are collected first:
+// warps that mixed them with full and empty cells ran that chain for one or two
+// lanes.  The flux kernels cover the cells whose fluxes reach the interior (the
+// interior across d, one cell beyond it along d), like the VOF sweeps, and take
+// the mixed ones from the VOF sweep's own list.  Built with -fmad=false so that each expression
 // keeps the Fortran operation order.
 //
 // Values the reference reads without setting are made definite: the
@@ -50,6 +53,9 @@ struct McArgs {
     const uint8_t* cg;    // c_mask of the fraction (Weymouth-Yue)
     double *m1, *m2, *m3; // momentum fluxes mom1 / mom2 / mom3
     const double* dxh;    // dxh by x index + ng
+    const long* list;     // the mixed flux cells (vof_sweep_list), their number and the list's room
+    const int* count;
+    long cap;
     Layout L;
     int d, scheme;
     double dt, dxyz, rho1, rho2;
@@ -57,14 +63,11 @@ struct McArgs {
 
 __host__ __device__ inline long dstride(const Layout& L, int d) { return d == 0 ? 1 : (d == 1 ? L.pitch : L.plane); }
 
-// (i, j, k), interior-relative, of a flux cell: the interior across d,
-// -1 .. n along d
-__device__ inline bool flux_cell(const Layout& L, int d, int& i, int& j, int& k) {
-    i = blockIdx.x * blockDim.x + threadIdx.x;
-    j = blockIdx.y;
-    k = blockIdx.z;
-    if (d == 0) i -= 1; else if (d == 1) j -= 1; else k -= 1;
-    return i <= L.n[0] && (d == 0 || i < L.n[0]);
+// layout index of flux cell t: the interior across d, -1 .. n along d, i fastest
+__device__ inline long flux_cell(const Layout& L, int d, unsigned t) {
+    const unsigned e0 = L.n[0] + (d == 0 ? 2 : 0), e1 = L.n[1] + (d == 1 ? 2 : 0);
+    const unsigned r = t / e0, k = r / e1;
+    return lidx(L, (int)(t - r * e0) - (d == 0), (int)(r - k * e1) - (d == 1), (int)k - (d == 2));
 }
 
 // (i, j, k), interior-relative, of element t of the ghosted array
@@ -160,36 +163,56 @@ __device__ __noinline__ double centroid_seg(const Plane P, int d, double lo, dou
 }
 
 // get_half_fractions of cvof along dir into w1 (lower half) and w2 (upper
-// half) over the [is-1, ie+1] box, zero elsewhere
-__global__ void k_mc_half(const double* __restrict__ c, double* __restrict__ w1, double* __restrict__ w2,
-                          const Layout L, int dir) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= L.total) return;
-    int i, j, k;
-    cell_of(L, t, i, j, k);
-    double h1 = 0.0, h2 = 0.0;
-    if (in_box(L, i, j, k)) {
-        const double cc = c[t];
-        h1 = cc;
-        h2 = cc;
-        if (cc > 0.0 && cc < 1.0) {
-            Plane P;
-            if (mc_fit_plane(c, L, t, dir, 0.0, 0.0, 0, &P)) {
-                h1 = 2.0 * fl3d_seg(P, dir, 0.0, 0.5);
-                h2 = 2.0 * fl3d_seg(P, dir, 0.5, 0.5);
-            }
+// half) over the [is-1, ie+1] box, zero elsewhere: the full and empty cells
+// here, the mixed ones into the list (one atomic add per block) for
+// k_mc_half_mixed.  One kernel for both ran at 16 warps per SM for the
+// registers of the plane fit: 29 us at 96^3, 14 us in two.
+__global__ void __launch_bounds__(256) k_mc_half(const double* __restrict__ c, double* __restrict__ w1,
+                                                 double* __restrict__ w2, long* __restrict__ list,
+                                                 int* __restrict__ count, long cap, const Layout L) {
+    __shared__ int n, room;
+    if (threadIdx.x == 0) n = 0;
+    __syncthreads();
+    const long t = blockIdx.x * 256L + threadIdx.x;
+    int e = -1;
+    if (t < L.total) {
+        int i, j, k;
+        cell_of(L, t, i, j, k);
+        const double cc = in_box(L, i, j, k) ? c[t] : 0.0;
+        w1[t] = cc;
+        w2[t] = cc;
+        if (cc > 0.0 && cc < 1.0) e = atomicAdd(&n, 1);
+    }
+    __syncthreads();
+    if (n == 0) return;
+    if (threadIdx.x == 0) room = atomicAdd(count, n);
+    __syncthreads();
+    if (e >= 0 && (long)room + e < cap) list[room + e] = t;
+}
+
+__global__ void __launch_bounds__(128) k_mc_half_mixed(const double* __restrict__ c, double* __restrict__ w1,
+                                                       double* __restrict__ w2, const long* __restrict__ list,
+                                                       const int* __restrict__ count, long cap, const Layout L,
+                                                       int dir) {
+    const long cnt = *count < cap ? *count : cap;
+    for (long q = blockIdx.x * 128L + threadIdx.x; q < cnt; q += gridDim.x * 128L) {
+        const long t = list[q];
+        Plane P;
+        if (mc_fit_plane(c, L, t, dir, 0.0, 0.0, 0, &P)) {
+            w1[t] = 2.0 * fl3d_seg(P, dir, 0.0, 0.5);
+            w2[t] = 2.0 * fl3d_seg(P, dir, 0.5, 0.5);
         }
     }
-    w1[t] = h1;
-    w2[t] = h2;
 }
 
 // the fraction and momentum of the control volumes over the box; the
-// fraction is cvof elsewhere, the momentum keeps its value elsewhere
+// fraction is cvof elsewhere, the momentum keeps its value elsewhere; cg is
+// c_mask of the fraction (vofmodules.f90:1295-1305), of which the sweeps read
+// the interior
 __global__ void k_mc_momentum(const double* __restrict__ cvof, const double* __restrict__ w1,
                               const double* __restrict__ w2, const double* __restrict__ us, double* __restrict__ tmp,
-                              double* __restrict__ mom, const Layout L, int dir, int staggered, double rho1,
-                              double rho2) {
+                              double* __restrict__ mom, uint8_t* __restrict__ cg, const Layout L, int dir,
+                              int staggered, double rho1, double rho2) {
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (t >= L.total) return;
     int i, j, k;
@@ -207,6 +230,7 @@ __global__ void k_mc_momentum(const double* __restrict__ cvof, const double* __r
         }
     }
     tmp[t] = tv;
+    cg[t] = tv > 0.5 ? 1 : 0;
 }
 
 // 0.5*(us(i) + us(i+e_dir)) wherever i+e_dir is in the array
@@ -216,19 +240,18 @@ __global__ void k_mc_face_avg(const double* __restrict__ us, double* __restrict_
     fv[t] = t + o2 < total ? 0.5 * (us[t] + us[t + o2]) : 0.0;
 }
 
-// CIAM momentum fluxes of one flux cell: swpzmom_stg (STAG; LIN: LinInterp)
-// or swpzmom
-template <bool STAG, bool LIN>
-__global__ void __launch_bounds__(128) k_mc_ciam_flux(const McArgs a) {
-    int i, j, k;
+// CIAM momentum fluxes of one flux cell n: swpzmom_stg (STAG; LIN: LinInterp)
+// or swpzmom; MIXED: only if 0 < c < 1, else only if not
+template <bool STAG, bool LIN, bool MIXED>
+__device__ __forceinline__ void mc_ciam_flux(const McArgs& a, long n) {
     const Layout& L = a.L;
-    if (!flux_cell(L, a.d, i, j, k)) return;
-    const long n = lidx(L, i, j, k), o = dstride(L, a.d);
+    const long o = dstride(L, a.d);
     const double* __restrict__ c = a.c;
     const double rho1 = a.rho1, rho2 = a.rho2;
     const int d = a.d;
     double a1, a2, uadv1 = 0.0, uadv3 = 0.0, uavg, u1 = 0.0, u2 = 0.0, u3 = 0.0;
     const double cc = c[n];
+    if ((cc > 0.0 && cc < 1.0) != MIXED) return;
     if (STAG) {
         a2 = a.fv[n] * a.dt / a.dxyz;
         a1 = a.fv[n - o] * a.dt / a.dxyz;
@@ -241,7 +264,7 @@ __global__ void __launch_bounds__(128) k_mc_ciam_flux(const McArgs a) {
         uadv1 = interpole3(u1, u2, u3, a.scheme, -0.5 - a1 / 2.0);
         uadv3 = interpole3(u1, u2, u3, a.scheme, 0.5 - a2 / 2.0);
     } else {
-        a2 = a.fv[n] * a.dt / a.dxh[i + L.ng];   // dxh(i) of the x index, as the reference writes it
+        a2 = a.fv[n] * a.dt / a.dxh[n % L.pitch];   // dxh(i) of the x index, as the reference writes it
         a1 = a.fv[n - o] * a.dt / a.dxyz;
     }
     const double mm1 = plic::dmax1(a1, 0.0);
@@ -249,7 +272,7 @@ __global__ void __launch_bounds__(128) k_mc_ciam_flux(const McArgs a) {
     if (STAG) uavg = interpole3(u1, u2, u3, a.scheme, (-plic::dmin1(a1, 0.0) - plic::dmax1(a2, 0.0)) / 2.0);
     else uavg = a.mom[n] / (rho2 * cc + rho1 * (1.0 - cc));
     double f1 = 0.0, f2 = 0.0, f3 = 0.0;
-    if (cc > 0.0 && cc < 1.0) {
+    if (MIXED) {
         Plane P;
         double vof;
         if (mc_fit_plane(c, L, n, d, a1, a2, 0, &P)) {
@@ -314,20 +337,19 @@ __global__ void __launch_bounds__(128) k_mc_ciam_flux(const McArgs a) {
     a.m3[n] = f3;
 }
 
-// Weymouth-Yue momentum fluxes of one flux cell: swprmom_stg (STAG; LIN:
-// LinInterp) or swprmom
-template <bool STAG, bool LIN>
-__global__ void __launch_bounds__(128) k_mc_wy_flux(const McArgs a) {
-    int i, j, k;
+// Weymouth-Yue momentum fluxes of one flux cell n: swprmom_stg (STAG; LIN:
+// LinInterp) or swprmom; MIXED as above
+template <bool STAG, bool LIN, bool MIXED>
+__device__ __forceinline__ void mc_wy_flux(const McArgs& a, long n) {
     const Layout& L = a.L;
-    if (!flux_cell(L, a.d, i, j, k)) return;
-    const long n = lidx(L, i, j, k), o = dstride(L, a.d);
+    const long o = dstride(L, a.d);
     const double* __restrict__ c = a.c;
     const double rho1 = a.rho1, rho2 = a.rho2;
     const int d = a.d;
+    const double cc = c[n];
+    if ((cc > 0.0 && cc < 1.0) != MIXED) return;
     const double a2 = a.fv[n] * a.dt / a.dxyz;
     const double a1 = a.fv[n - o] * a.dt / a.dxyz;
-    const double cc = c[n];
     double uadv1, uadv3, u1 = 0.0, u2 = 0.0, u3 = 0.0;
     if (STAG) {
         const double ro1 = (rho2 * c[n - o] + rho1 * (1.0 - c[n - o]));
@@ -342,7 +364,7 @@ __global__ void __launch_bounds__(128) k_mc_wy_flux(const McArgs a) {
         uadv1 = uadv3 = a.mom[n] / (rho2 * cc + rho1 * (1.0 - cc));
     }
     double f1 = 0.0, f3 = 0.0;
-    if (cc > 0.0 && cc < 1.0) {
+    if (MIXED) {
         Plane P;
         double vof;
         mc_plane_wy(c, L, n, &P);
@@ -390,6 +412,39 @@ __global__ void __launch_bounds__(128) k_mc_wy_flux(const McArgs a) {
     }
     a.m1[n] = f1;
     a.m3[n] = f3;
+}
+
+// The fluxes of the F flux cells: MIXED, the listed mixed ones, every lane one;
+// else the full and empty cells, one after another across rows.  (A cell above 1
+// is in the VOF sweep's list but takes the closed form here.)  Apart, because
+// the plane fit holds 128 registers: one kernel for all, cells as they lie, took
+// 48 us at 96^3 with 24 drops; one kernel with the mixed cells in blocks of their
+// own 29 us; two kernels 17 us.
+template <bool WY, bool STAG, bool LIN, bool MIXED>
+__global__ void __launch_bounds__(128) k_mc_flux(const McArgs a, unsigned F) {
+    if (MIXED) {
+        const long cnt = *a.count < a.cap ? *a.count : a.cap;
+        for (long q = blockIdx.x * 128L + threadIdx.x; q < cnt; q += gridDim.x * 128L) {
+            if (WY) mc_wy_flux<STAG, LIN, true>(a, a.list[q]);
+            else mc_ciam_flux<STAG, LIN, true>(a, a.list[q]);
+        }
+    } else {
+        const unsigned t = blockIdx.x * 128u + threadIdx.x;
+        if (t >= F) return;
+        const long n = flux_cell(a.L, a.d, t);
+        if (WY) mc_wy_flux<STAG, LIN, false>(a, n);
+        else mc_ciam_flux<STAG, LIN, false>(a, n);
+    }
+}
+
+template <bool WY, bool STAG, bool LIN>
+int mc_fluxes(paris_ctx* c, const McArgs& a) {
+    const Layout& L = a.L;
+    const long F = (long)(L.n[0] + (a.d == 0 ? 2 : 0)) * (L.n[1] + (a.d == 1 ? 2 : 0)) * (L.n[2] + (a.d == 2 ? 2 : 0));
+    const char* name = WY ? "mc_wy_flux" : "mc_ciam_flux";
+    PARIS_LAUNCH_N(c, name, 0L, (k_mc_flux<WY, STAG, LIN, true>), c->nsm * 4, 128, 0, a, (unsigned)F);
+    PARIS_LAUNCH_N(c, name, c->N, (k_mc_flux<WY, STAG, LIN, false>), div_up(F, 128), 128, 0, a, (unsigned)F);
+    return PARIS_OK;
 }
 
 // the momentum of the interior after the sweep along d
@@ -491,11 +546,6 @@ __global__ void k_mc_velocity_cen(const double* __restrict__ tmp, const double* 
         der[t] = ((mom[t] / r0 + mom[t + o2] / r1) * 0.5 - us[t]) / dt;
 }
 
-__global__ void k_mc_copy_i8(int8_t* __restrict__ dst, const int8_t* __restrict__ src, long total) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t < total) dst[t] = src[t];
-}
-
 }  // namespace
 
 // SetMomentumBC for the wall faces of the grid, then nothing else: the
@@ -554,6 +604,7 @@ extern "C" int paris_vof_mom_sweeps(paris_handle_t c, int32_t tswap, double dt, 
         PARIS_CHECK(ctx_alloc_field(c, f));
     PARIS_CHECK(ctx_alloc_field(c, PARIS_FIELD_VOF_FLAG));
     PARIS_CHECK(mc_alloc(c));
+    PARIS_CHECK(vof_scratch(c));
     const Layout& L = c->L;
     const long nt = L.total;
     WallV WV;
@@ -575,18 +626,19 @@ extern "C" int paris_vof_mom_sweeps(paris_handle_t c, int32_t tswap, double dt, 
         double* tmp = c->mc_tmp;
         // 1. the control volumes: fraction and momentum
         if (staggered) {
-            PARIS_LAUNCH_N(c, "mc_half_fractions", nt, k_mc_half, gb, 256, 0, cvof, w1, w2, L, dir);
-            PARIS_CHECK(ctx_ghost_fill(c, w1));
-            PARIS_CHECK(ctx_ghost_fill(c, w2));
+            PARIS_CUDA_TRY(c, cudaMemsetAsync(c->mixsegn, 0, sizeof(int), c->stream));
+            PARIS_LAUNCH_N(c, "mc_half_fractions", nt, k_mc_half, gb, 256, 0, cvof, w1, w2, c->mixlist, c->mixsegn,
+                           c->mixcap, L);
+            PARIS_LAUNCH_N(c, "mc_half_fractions", 0L, k_mc_half_mixed, c->nsm * 4, 128, 0, cvof, w1, w2, c->mixlist,
+                           c->mixsegn, c->mixcap, L, dir);
+            PARIS_CHECK(ctx_ghost_fill(c, us, w1, w2));
+        } else {
+            PARIS_CHECK(ctx_ghost_fill(c, us));
         }
-        PARIS_CHECK(ctx_ghost_fill(c, us));
-        PARIS_LAUNCH_N(c, "mc_momentum", nt, k_mc_momentum, gb, 256, 0, cvof, w1, w2, us, tmp, mom, L, dir,
+        PARIS_LAUNCH_N(c, "mc_momentum", nt, k_mc_momentum, gb, 256, 0, cvof, w1, w2, us, tmp, mom, c->mc_cg, L, dir,
                        staggered, c->d.rho1, c->d.rho2);
         if (staggered) PARIS_CHECK(mc_wall_bc(c, mom, us, cvof, dir, WV));
-        PARIS_CHECK(ctx_ghost_fill(c, tmp));
-        PARIS_CHECK(ctx_ghost_fill(c, mom));
-        PARIS_LAUNCH(c, k_mc_copy_i8, gb, 256, 0, c->mc_flag, c->flag, nt);
-        if (wy) PARIS_LAUNCH(c, k_c_mask, gb, 256, 0, tmp, c->mc_cg, nt);
+        PARIS_CHECK(ctx_ghost_fill(c, tmp, mom));
         // 2. the three split sweeps of momentum and fraction
         for (int s = 0; s < 3; s++) {
             const int d = order[s];
@@ -612,22 +664,19 @@ extern "C" int paris_vof_mom_sweeps(paris_handle_t c, int32_t tswap, double dt, 
             a.dxyz = c->h_dxh[g];
             a.rho1 = c->d.rho1;
             a.rho2 = c->d.rho2;
-            int ext[3] = {L.n[0], L.n[1], L.n[2]};
-            ext[d] += 2;
-            const dim3 fg(div_up(ext[0], 128), ext[1], ext[2]), ig(div_up(L.n[0], 128), L.n[1], L.n[2]);
-            if (wy) {
-                if (staggered && lin_interp) PARIS_LAUNCH_N(c, "mc_wy_flux", c->N, (k_mc_wy_flux<true, true>), fg, 128, 0, a);
-                else if (staggered) PARIS_LAUNCH_N(c, "mc_wy_flux", c->N, (k_mc_wy_flux<true, false>), fg, 128, 0, a);
-                else PARIS_LAUNCH_N(c, "mc_wy_flux", c->N, (k_mc_wy_flux<false, false>), fg, 128, 0, a);
-                if (staggered) PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<true, true>), ig, 128, 0, a);
-                else PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<true, false>), ig, 128, 0, a);
-            } else {
-                if (staggered && lin_interp)
-                    PARIS_LAUNCH_N(c, "mc_ciam_flux", c->N, (k_mc_ciam_flux<true, true>), fg, 128, 0, a);
-                else if (staggered) PARIS_LAUNCH_N(c, "mc_ciam_flux", c->N, (k_mc_ciam_flux<true, false>), fg, 128, 0, a);
-                else PARIS_LAUNCH_N(c, "mc_ciam_flux", c->N, (k_mc_ciam_flux<false, false>), fg, 128, 0, a);
-                PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<false, false>), ig, 128, 0, a);
-            }
+            PARIS_CHECK(vof_sweep_list(c, d, tmp));
+            a.list = c->mixlist;
+            a.count = c->mixsegn;
+            a.cap = c->mixcap;
+            const dim3 ig(div_up(L.n[0], 128), L.n[1], L.n[2]);
+            const int form = !staggered ? 0 : (lin_interp ? 2 : 1);
+            if (wy) PARIS_CHECK((form == 2 ? mc_fluxes<true, true, true> : form ? mc_fluxes<true, true, false>
+                                                                                : mc_fluxes<true, false, false>)(c, a));
+            else PARIS_CHECK((form == 2 ? mc_fluxes<false, true, true> : form ? mc_fluxes<false, true, false>
+                                                                              : mc_fluxes<false, false, false>)(c, a));
+            if (!wy) PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<false, false>), ig, 128, 0, a);
+            else if (staggered) PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<true, true>), ig, 128, 0, a);
+            else PARIS_LAUNCH_N(c, "mc_update", c->N, (k_mc_update<true, false>), ig, 128, 0, a);
             // SetMomentumBC after the sweep (the momentum of component d for
             // the CIAM and centred sweeps; swprmom_stg passes dir when dir is
             // x or d is y or z, and none otherwise), then do_all_ghost(mom)

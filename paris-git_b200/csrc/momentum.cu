@@ -699,8 +699,6 @@ extern "C" int paris_set_velocity_bc(paris_handle_t c, const double* wall_vel) {
                        c->fld[PARIS_FIELD_U], c->fld[PARIS_FIELD_V], c->fld[PARIS_FIELD_W], c->L, dir, lo, hi, WV);
     }
     // do_ghost_vector: the periodic images
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_U]));
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_V]));
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_W]));
+    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_U], c->fld[PARIS_FIELD_V], c->fld[PARIS_FIELD_W]));
     return PARIS_OK;
 }

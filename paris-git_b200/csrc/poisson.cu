@@ -319,8 +319,6 @@ extern "C" int paris_project_velocity(paris_handle_t c, double dt) {
     PARIS_LAUNCH_N(c, "project_velocity", c->N, k_project, cell_grid(c->L), cell_block(), 0, c->fld[PARIS_FIELD_U], c->fld[PARIS_FIELD_V],
                  c->fld[PARIS_FIELD_W], c->fld[PARIS_FIELD_P], c->fld[PARIS_FIELD_RHO], c->L, c->bnd, metric(c), dt);
     // SetVelocityBC + do_ghost_vector follow the projection (paris.f90:590-591)
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_U]));
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_V]));
-    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_W]));
+    PARIS_CHECK(ctx_ghost_fill(c, c->fld[PARIS_FIELD_U], c->fld[PARIS_FIELD_V], c->fld[PARIS_FIELD_W]));
     return PARIS_OK;
 }

@@ -282,16 +282,12 @@ __global__ void k_c_mask(const double* __restrict__ c, uint8_t* __restrict__ cg,
 }
 
 // scratch of the sweeps, allocated with the handle (paris_gpu_init): the
-// sparse flux arrays and the segmented list (sized for the largest flux
-// domain of the three directions)
+// sparse flux arrays and the list of mixed cells (room for the interior and one
+// ghost layer, which holds the flux domain of each direction)
 int vof_scratch(paris_ctx* c) {
     const Layout& L = c->L;
     if (c->vflux) return PARIS_OK;
-    long F = 0;
-    for (int d = 0; d < 3; d++) {
-        long e = (long)(L.n[0] + (d == 0 ? 2 : 0)) * (L.n[1] + (d == 1 ? 2 : 0)) * (L.n[2] + (d == 2 ? 2 : 0));
-        F = e > F ? e : F;
-    }
+    const long F = (long)(L.n[0] + 2) * (L.n[1] + 2) * (L.n[2] + 2);
     PARIS_CUDA_TRY(c, cudaMalloc(&c->vflux, 3 * L.total * sizeof(double)));
     PARIS_CUDA_TRY(c, cudaMalloc(&c->mixlist, F * sizeof(long)));
     PARIS_CUDA_TRY(c, cudaMalloc(&c->mixsegn, sizeof(int)));
@@ -299,10 +295,27 @@ int vof_scratch(paris_ctx* c) {
     return PARIS_OK;
 }
 
+// the mixed flux cells of a sweep of src along d, into c->mixlist and *c->mixsegn
+int vof_sweep_list(paris_ctx* c, int d, const double* src) {
+    const Layout& L = c->L;
+    PARIS_CHECK(vof_scratch(c));
+    SweepArgs a{};
+    a.c = src;
+    a.list = c->mixlist;
+    a.count = c->mixsegn;
+    a.cap = c->mixcap;
+    a.L = L;
+    a.d = d;
+    const long F = (long)(L.n[0] + (d == 0 ? 2 : 0)) * (L.n[1] + (d == 1 ? 2 : 0)) * (L.n[2] + (d == 2 ? 2 : 0));
+    PARIS_CUDA_TRY(c, cudaMemsetAsync(c->mixsegn, 0, sizeof(int), c->stream));
+    PARIS_LAUNCH_N(c, "vof_sweep", 0L, k_vof_mixed_list, div_up(F, kVofSeg), kVofListThreads, 0, a, (unsigned)F);
+    return PARIS_OK;
+}
+
+// the sweep of src along d from the list that vof_sweep_list left
 int vof_sweep_dir(paris_ctx* c, int d, double dt, const double* src, double* dst, int8_t* flag, const double* us,
                   const uint8_t* cg) {
     const Layout& L = c->L;
-    PARIS_CHECK(vof_scratch(c));
     SweepArgs a;
     a.c = src;
     a.cn = dst;
@@ -323,11 +336,8 @@ int vof_sweep_dir(paris_ctx* c, int d, double dt, const double* src, double* dst
     int ex;
     a.rdxyz = frexp(a.dxyz, &ex) == 0.5 ? 1.0 / a.dxyz : 0.0;   // 1/2^k is exact
     a.epsc = c->d.epsc;
-    const long F = (long)(L.n[0] + (d == 0 ? 2 : 0)) * (L.n[1] + (d == 1 ? 2 : 0)) * (L.n[2] + (d == 2 ? 2 : 0));
     // the four kernels of a direction share the profile label "vof_sweep",
     // with the direction's cells counted once (on the update)
-    PARIS_CUDA_TRY(c, cudaMemsetAsync(c->mixsegn, 0, sizeof(int), c->stream));
-    PARIS_LAUNCH_N(c, "vof_sweep", 0L, k_vof_mixed_list, div_up(F, kVofSeg), kVofListThreads, 0, a, (unsigned)F);
     PARIS_LAUNCH_N(c, "vof_sweep", 0L, k_vof_mixed_flux, c->nsm * 16, 128, 0, a);
     const unsigned across = div_up(L.n[0], kVofUpdThreads * kVofUpd);
     const unsigned bw = 32 * div_up(div_up(L.n[0], (long)across * kVofUpd), 32);
@@ -339,6 +349,7 @@ int vof_sweep_dir(paris_ctx* c, int d, double dt, const double* src, double* dst
 }
 
 static int sweep(paris_ctx* c, int d, double dt) {
+    PARIS_CHECK(vof_sweep_list(c, d, c->fld[PARIS_FIELD_CVOF]));
     PARIS_CHECK(vof_sweep_dir(c, d, dt, c->fld[PARIS_FIELD_CVOF], c->c2, c->flag, c->fld[PARIS_FIELD_U + d], c->cg));
     double* t = c->fld[PARIS_FIELD_CVOF];
     c->fld[PARIS_FIELD_CVOF] = c->c2;
