@@ -166,7 +166,7 @@ __device__ __noinline__ double centroid_seg(const Plane P, int d, double lo, dou
 // half) over the [is-1, ie+1] box, zero elsewhere: the full and empty cells
 // here, the mixed ones into the list (one atomic add per block) for
 // k_mc_half_mixed.  One kernel for both ran at 16 warps per SM for the
-// registers of the plane fit: 29 us at 96^3, 14 us in two.
+// registers of the plane fit: 29 us at 96^3, 18 us in two.
 __global__ void __launch_bounds__(256) k_mc_half(const double* __restrict__ c, double* __restrict__ w1,
                                                  double* __restrict__ w2, long* __restrict__ list,
                                                  int* __restrict__ count, long cap, const Layout L) {
@@ -419,7 +419,7 @@ __device__ __forceinline__ void mc_wy_flux(const McArgs& a, long n) {
 // is in the VOF sweep's list but takes the closed form here.)  Apart, because
 // the plane fit holds 128 registers: one kernel for all, cells as they lie, took
 // 48 us at 96^3 with 24 drops; one kernel with the mixed cells in blocks of their
-// own 29 us; two kernels 17 us.
+// own 29 us; two kernels 22 us together.
 template <bool WY, bool STAG, bool LIN, bool MIXED>
 __global__ void __launch_bounds__(128) k_mc_flux(const McArgs a, unsigned F) {
     if (MIXED) {

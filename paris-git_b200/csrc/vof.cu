@@ -203,10 +203,11 @@ __device__ inline double cell_flux(const SweepArgs& a, double cc, long n, double
 
 // 3. the update of the interior: new c, clipping (swpz :224-230 / swpr
 // :731-745 and get_flags_and_clip) and the flag, into the second buffer.
-// Each thread updates kVofUpd cells of a row, a block's width apart (a width
-// that covers the row with few idle lanes: 150 cells in two of 96 instead of two
-// of 128 with half the warps idle); the volume fractions and face velocities of all of them are loaded before any
-// test on them, so their loads are in flight together.
+// Each thread updates kVofUpd cells of a row, a block's width apart; the width
+// covers the row with few idle lanes (150 cells: one block of 96 threads, 215 to
+// 198 us for three sweeps of 150x93x121).  The volume fractions and face
+// velocities of all its cells are loaded before any test on them, so their loads
+// are in flight together.
 static constexpr int kVofUpdThreads = 128, kVofUpd = 2;
 __global__ void __launch_bounds__(kVofUpdThreads) k_vof_update(const SweepArgs a) {
     const int j = blockIdx.y, k = blockIdx.z, bw = blockDim.x;
