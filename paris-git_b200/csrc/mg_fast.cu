@@ -850,24 +850,15 @@ static int sweep_tma_chunk(paris_ctx* c, const FastLevel<float>& l) {
     return (int)div_up(l.n[2], nbz);
 }
 
-// Launch geometry of the column sweep with configuration C on level l: tiles
-// as wide as the grid where its chunks fit a staged row, else equal tiles with
-// one ring chunk on either side; planes per block (even) so that the blocks
-// fill whole waves of the C::MINB x nsm resident ones with long chunks (a
-// chunk takes about three planes' time before its first output).
+// Launch geometry of the column sweep with configuration C on level l: planes
+// per block (even) so that the blocks fill whole waves of the C::MINB x nsm
+// resident ones with long chunks (a chunk takes about three planes' time before
+// its first output).
 template <class C>
 static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l) {
-    const int n0 = l.n[0], n2 = l.n[2], V = C::VEC;
+    const int n0 = l.n[0], n2 = l.n[2];
     SwColGeo g;
-    if (n0 / V <= C::PITCH) {
-        g.W = n0;
-        g.H = 0;
-    } else {
-        const int t = (int)div_up(n0, (C::PITCH - 2) * V);
-        g.W = (int)div_up(div_up(n0, t), V) * V;
-        g.H = V;
-    }
-    g.lanes = (g.W + 2 * g.H) / V;
+    sweep_col_tiles<C>(n0, g);
     const long tiles = (long)div_up(n0, g.W) * div_up(l.n[1], C::TY), slots = (long)C::MINB * c->nsm;
     double best = -1.0;
     g.zc = n2;

@@ -16,11 +16,14 @@
 // plane k-1, which is final and stored:
 //   - the iterate of the thread's own cells at planes k-2..k+1 and the
 //     coefficients of its S cells at plane k-1 stay in registers; the rows
-//     around come from shared memory as 16-byte loads, the cells left and right
-//     as one scalar each;
-//   - F of plane k reads only S cells, which no thread writes in that step, and
-//     S of plane k-1 reads F cells written a step earlier, so one barrier per
-//     plane orders everything;
+//     around come from shared memory, the cells left and right as one scalar
+//     each;
+//   - F of plane k reads S cells from the staged iterate, which is not written
+//     again once a step has begun to read it; the new F values go to a ring of
+//     their own, U = VEC / 2 of them a chunk, where S of plane k reads them a
+//     step later.  No step reads what it writes, so one barrier per plane orders
+//     everything (a ring of its own also holds no S cells, which S has in
+//     registers: half the bytes per row that S reads);
 //   - the cells a thread updates are the same half of its chunk in both
 //     colours, by the parity of its row and plane.  Rows are dealt to warps
 //     even rows first, so a warp takes one parity and runs its steps in pairs
@@ -56,11 +59,12 @@ struct SwColCfg {
     static constexpr int VEC = 16 / (int)sizeof(T);
     static constexpr int EV = (TY + 3) / 2, OD = (TY + 2) / 2;               // even and odd rows of 0..TY+1
     static constexpr int NE = (EV * PITCH + 31) / 32 * 32, NT = NE + (OD * PITCH + 31) / 32 * 32;
-    static constexpr int XS = D + 3, CS = D + 1;                             // planes in the rings
+    static constexpr int XS = D + 2, CS = D + 1;                             // planes in the rings
     static constexpr uint32_t ROW = PITCH * 16, XSLOT = ROW * (TY + 4);
+    static constexpr uint32_t NROW = PITCH * 8, NSLOT = NROW * (TY + 4);     // new F cells: rows y0-2..y0+TY+1, of which S uses y0-1..y0+TY
     static constexpr uint32_t O_CY = ROW * (TY + 2), O_CZ = O_CY + ROW * (TY + 3), O_B = O_CZ + ROW * (TY + 2);
     static constexpr uint32_t CSLOT = O_B + ROW * (TY + 2);
-    static constexpr size_t SMEM = (size_t)XSLOT * XS + (size_t)CSLOT * CS;
+    static constexpr size_t SMEM = (size_t)XSLOT * XS + (size_t)CSLOT * CS + 2 * (size_t)NSLOT;
     static_assert(SMEM <= 227 * 1024 && NT <= 1024, "one block fits an SM");
     static_assert(EV >= 3, "the first three rows of threads stage the rows only read");
 };
@@ -76,6 +80,22 @@ struct alignas(16) SwChunk {
 struct SwColGeo {
     int W, H, lanes, zc;
 };
+
+// the tiles across a row of n0 cells: as wide as the grid where its chunks fit
+// a staged row, else equal tiles with one ring chunk on either side
+template <class C>
+inline void sweep_col_tiles(int n0, SwColGeo& g) {
+    const int V = C::VEC;
+    if (n0 / V <= C::PITCH) {
+        g.W = n0;
+        g.H = 0;
+    } else {
+        const int t = (n0 + (C::PITCH - 2) * V - 1) / ((C::PITCH - 2) * V);
+        g.W = ((n0 + t - 1) / t + V - 1) / V * V;
+        g.H = V;
+    }
+    g.lanes = (g.W + 2 * g.H) / V;
+}
 
 template <class C, bool ZERO, bool CORR>
 __global__ void __launch_bounds__(C::NT, C::MINB)
@@ -115,12 +135,23 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
     const uint32_t oe = ROW * (q == 1 ? TY + 3 : 0) + 16u * lane;     // its chunk of the rows only read
     const uint32_t s_x = (uint32_t)__cvta_generic_to_shared(sw_raw);
     constexpr uint32_t C0 = XS * C::XSLOT;                            // the coefficient ring starts here
+    constexpr uint32_t N0 = C0 + CS * C::CSLOT;                       // and the two planes of new F cells here
+    constexpr uint32_t NB = U * sizeof(T);
+    const uint32_t fo = C::NROW * (r + 1) + NB * lane;               // the thread's F cells in a plane of them
     // the cells left and right of the chunk: across a seam in a whole row, absent (zero) at a wall
     const bool whole = g.H == 0;
     const bool wz = whole && lane == 0 && !B.per[0], ez = whole && lane == g.lanes - 1 && !B.per[0];
     const uint32_t ow = o + (lane > 0 ? -(int)sizeof(T) : (whole ? g.lanes * 16 - (int)sizeof(T) : 0));
     const uint32_t oea = o + (lane < g.lanes - 1 ? 16 : (whole ? 16 - g.lanes * 16 : 16 - (int)sizeof(T)));
 
+    // the F cell left (the last of a chunk's) and right (the first) of the chunk
+    const uint32_t fow = fo + (lane > 0 ? -(int)sizeof(T) : (whole ? g.lanes * (int)NB - (int)sizeof(T) : 0));
+    const uint32_t foe = fo + (lane < g.lanes - 1 ? (int)NB : (whole ? (int)NB - g.lanes * (int)NB : 0));
+
+    struct alignas(U * sizeof(T)) Half {
+        T v[U];
+    };
+    auto ldh = [](uint32_t a) { return *reinterpret_cast<const Half*>(sw_raw + a); };
     auto ldc = [](uint32_t a) { return *reinterpret_cast<const Chunk*>(sw_raw + a); };   // a: offset from sw_raw
     auto lds = [](uint32_t a) { return *reinterpret_cast<const T*>(sw_raw + a); };
     const bool pz = B.per[2];
@@ -155,6 +186,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
             st0(s + C::O_CZ);
             st0(s + C::O_B);
         }
+        for (int d = 0; d < 2; d++) *reinterpret_cast<Half*>(sw_raw + N0 + d * C::NSLOT + fo) = Half{};
     }
     if (eon && !eok) {
         for (int d = 0; d < XS; d++)
@@ -167,9 +199,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
     // staged, fetched a plane ahead.  Neighbours read iterate plane k+1 from
     // step k+1 on, so step k adds it after its barrier; plane z0-1 gets it
     // before the first one.
-    struct alignas(U * sizeof(T)) Half {
-        T v[U];
-    };
     const uint32_t cn0 = (uint32_t)n0 >> 1, cplane = cn0 * ((uint32_t)n1 >> 1);
     const uint32_t coff = ok ? ((uint32_t)wi >> 1) + cn0 * ((uint32_t)wj >> 1) : 0u;
     const uint32_t ecoff = ex ? ((uint32_t)wi >> 1) + cn0 * ((uint32_t)ej >> 1) : 0u;
@@ -220,11 +249,13 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
     uint32_t xo = (uint32_t)gi0 + (uint32_t)n0 * (uint32_t)j + plane * (uint32_t)(z0 - 3);   // the chunk at plane k-1 once advanced (mod 2^32)
     double bx = 0.0;
     const T w = v.omega;
-    // byte offsets of the slots of iterate planes k-2, k-1, k and coefficient
-    // planes k-1, k.  The planes staged at step k, k+1+D and k+D, take the
-    // slots of planes k-2 and k-1, last read in step k-1.
-    uint32_t x2m = (XS - 2) * C::XSLOT, xm = (XS - 1) * C::XSLOT, xk = 0;
+    // byte offsets of the slots of iterate and coefficient planes k-1, k, and of
+    // the new F cells of planes k-1, k.  The planes staged at step k, k+1+D and
+    // k+D, take the slots of planes k-1, and the F cells of plane k those of
+    // plane k-2: last read in step k-1.
+    uint32_t xm = (XS - 1) * C::XSLOT, xk = 0;
     uint32_t cm = C0 + (CS - 1) * C::CSLOT, ck = C0;
+    uint32_t nm = N0 + C::NSLOT, nk = N0;
 
     auto step = [&](auto PC, int k) {   // PC: parity of the updated cells of the chunk
         constexpr int P = decltype(PC)::value;
@@ -243,7 +274,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         }
         __syncthreads();
         if (k + D <= z1) {
-            stage_x(k + 1 + D, x2m);
+            stage_x(k + 1 + D, xm);
             stage_c(k + D, cm);
         }
         cp_async_commit();
@@ -256,9 +287,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         if (!ZERO) {
             if (k == z0 - 1 && in) x1 = ldc(fx + ROW);
             if (inside(k + 1)) {
-                x2 = ldc(xp + o + ROW);
+                if (!CORR) x2 = ldc(xp + o + ROW);
                 if (CORR) {
-                    if (ok) {
+                    if (ok) {   // (another thread's chunk is still being added to)
+                        x2 = ldc(xp + o + ROW);
 #pragma unroll
                         for (int e = 0; e < VEC; e++) x2.v[e] += cown.v[e >> 1];
                         *reinterpret_cast<Chunk*>(sw_raw + xp + o + ROW) = x2;
@@ -287,11 +319,15 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
                                 xn.v[e], xb.v[e], x2.v[e], b.v[e], x1.v[e], w, t) && fok)
                 nx.v[e] = t;
         }
-        if (fok) *reinterpret_cast<Chunk*>(sw_raw + fx + ROW) = nx;
+        if (ok) {   // (zero where plane k is outside a wall)
+            Half nf;
+#pragma unroll
+            for (int u = 0; u < U; u++) nf.v[u] = nx.v[P + 2 * u];
+            *reinterpret_cast<Half*>(sw_raw + nk + fo) = nf;
+        }
         // S at plane k-1, final: stored
-        const uint32_t fm = xm + o;
-        const Chunk ps = ldc(fm), pn = ldc(fm + 2 * ROW);
-        T pl = lds(xm + ROW + (P == 0 ? ow : oea));
+        const Half ps = ldh(nm + fo - C::NROW), pn = ldh(nm + fo + C::NROW);
+        T pl = lds(nm + (P == 0 ? fow : foe));
         if (P == 0 ? wz : ez) pl = (T)0;
         Chunk ns = xb;
 #pragma unroll
@@ -299,7 +335,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
             const int e = P + 2 * u;
             T t;
             if (SwUpd<T>::apply(a1[u], a2[u], a3[u], a4[u], a5[u], a6[u], e > 0 ? xb.v[e > 0 ? e - 1 : 0] : pl,
-                                e < L ? xb.v[e < L ? e + 1 : 0] : pl, ps.v[e], pn.v[e], xa.v[e], nx.v[e], bb.v[e],
+                                e < L ? xb.v[e < L ? e + 1 : 0] : pl, ps.v[u], pn.v[u], xa.v[e], nx.v[e], bb.v[e],
                                 xb.v[e], w, t))
                 ns.v[e] = t;
         }
@@ -327,9 +363,11 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         xa = xb;
         xb = nx;
         x1 = x2;
-        x2m = xm;
         xm = xk;
         xk = xp;
+        const uint32_t nt = nm;
+        nm = nk;
+        nk = nt;
         cm = ck;
         ck = ck == C0 + (CS - 1) * C::CSLOT ? C0 : ck + C::CSLOT;
     };
