@@ -61,7 +61,7 @@ __device__ inline void west_coefs(const LV<T>& v, const Bnd& B, int i, int j, in
 }
 
 template <typename T>
-__device__ inline void nbrs(const LV<T>& v, const T* __restrict__ x, const Bnd& B, int i, int j, int k, long m, T& xw,
+__device__ inline void nbrs(const LV<T>& v, const T* x, const Bnd& B, int i, int j, int k, long m, T& xw,
                             T& xe, T& xs, T& xn, T& xb, T& xt) {
     long sy = v.n0, sz = (long)v.n0 * v.n1;
     xw = i > 0 ? x[m - 1] : (B.per[0] ? x[m + v.n0 - 1] : (T)0);
@@ -84,12 +84,60 @@ __device__ inline void smooth_cell(const LV<T>& v, const Bnd& B, int i, int j, i
     if (d > (T)0) v.x[m] = relax(s / d, v.omega != (T)1 ? v.x[m] : (T)0, v.omega);
 }
 
+// A periodic axis with an odd number of cells (on the coarsest level only)
+// joins cells of one colour: its first and its last.  A pass over them all at
+// once would read values that it is writing; so a colour pass takes the cells
+// in no such last plane first, then those in one, in two and in three.  Two
+// neighbours of one colour differ by one in that count, and the last plane
+// comes after the first as in the loop order i, j, k: the pass in that order,
+// to the bit.
+__device__ inline int seam_count(const Bnd& B, int n0, int n1, int n2, int i, int j, int k) {
+    return (B.per[0] && (n0 & 1) && i == n0 - 1) + (B.per[1] && (n1 & 1) && j == n1 - 1) +
+           (B.per[2] && (n2 & 1) && k == n2 - 1);
+}
+__host__ __device__ inline int seam_axes(const Bnd& B, int n0, int n1, int n2) {
+    return (B.per[0] && (n0 & 1)) + (B.per[1] && (n1 & 1)) + (B.per[2] && (n2 & 1));
+}
+// f(i, j, k) for the cells of the colour in `count` such planes, dealt to st threads
+template <typename F>
+__device__ inline void for_seam_cells(const Bnd& B, int n0, int n1, int n2, int color, int count, int t0, int st, F f) {
+    const bool s0 = B.per[0] && (n0 & 1), s1 = B.per[1] && (n1 & 1), s2 = B.per[2] && (n2 & 1);
+    const int p0 = s0 ? n1 * n2 : 0, p1 = s1 ? n0 * n2 : 0, p2 = s2 ? n0 * n1 : 0;
+    for (int t = t0; t < p0 + p1 + p2; t += st) {
+        int i, j, k;
+        if (t < p0) {
+            i = n0 - 1; k = t / n1; j = t - k * n1;
+        } else if (t < p0 + p1) {
+            const int q = t - p0;
+            j = n1 - 1; k = q / n0; i = q - k * n0;
+            if (s0 && i == n0 - 1) continue;   // (in the planes before)
+        } else {
+            const int q = t - p0 - p1;
+            k = n2 - 1; j = q / n0; i = q - j * n0;
+            if ((s0 && i == n0 - 1) || (s1 && j == n1 - 1)) continue;
+        }
+        if (((i + j + k + color) & 1) == 0 && seam_count(B, n0, n1, n2, i, j, k) == count) f(i, j, k);
+    }
+}
+
 // grid (ceil(n/128), n1, n2), block 128: one thread per cell of the colour
-template <typename T>
+// (SEAM: but those in a last plane of a periodic axis with an odd extent)
+template <typename T, bool SEAM>
 __global__ void k_fast_smooth(const LV<T> v, const Bnd B, int color) {
     int ih = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
     int i = 2 * ih + ((j + k + color) & 1);
-    if (i < v.n0) smooth_cell(v, B, i, j, k);
+    if (i < v.n0 && !(SEAM && seam_count(B, v.n0, v.n1, v.n2, i, j, k))) smooth_cell(v, B, i, j, k);
+}
+
+// the rest of a SEAM pass, one block
+template <typename T>
+__global__ void __launch_bounds__(1024) k_fast_smooth_seam(const LV<T> v, const Bnd B, int color) {
+    const int axes = seam_axes(B, v.n0, v.n1, v.n2);
+    for (int count = 1; count <= axes; count++) {
+        for_seam_cells(B, v.n0, v.n1, v.n2, color, count, threadIdx.x, blockDim.x,
+                       [&](int i, int j, int k) { smooth_cell(v, B, i, j, k); });
+        __syncthreads();
+    }
 }
 
 // Residual and restriction with one warp per 32 coarse cells of a fine row:
@@ -185,8 +233,8 @@ __device__ inline int div_small(int t, int d, float rd) {
 // The V-cycle from level L0 (at most 16^3 cells) down to the coarsest in one
 // block, every level held in the block's shared memory and addressed by element
 // offsets from one shared array (shared-memory loads rather than generic ones),
-// the neighbours of a cell taken branch-free (the wrapped or clamped index always
-// loaded, the value dropped at a wall), the cell indices of each thread
+// the neighbours of a cell taken branch-free (at a wall the cell itself is
+// loaded and the value dropped), the cell indices of each thread
 // decomposed once per pass, and the restriction split into a pass over the
 // fine cells (their residuals into a scratch array) and one over the coarse
 // cells (the 8 residuals summed with i fastest).
@@ -204,18 +252,20 @@ __device__ inline CcNb cc_nb(const CcLvl& l, const Bnd& B, int i, int j, int k) 
     const int n0 = l.n0, n1 = l.n1, n2 = l.n2, sy = n0, sz = n0 * n1;
     CcNb q;
     q.m = i + sy * j + sz * k;
-    q.mw = i > 0 ? q.m - 1 : q.m + n0 - 1;
-    q.me = i < n0 - 1 ? q.m + 1 : q.m - (n0 - 1);
-    q.ms = j > 0 ? q.m - sy : q.m + sy * (n1 - 1);
-    q.mn = j < n1 - 1 ? q.m + sy : q.m - sy * (n1 - 1);
-    q.mb = k > 0 ? q.m - sz : q.m + sz * (n2 - 1);
-    q.mt = k < n2 - 1 ? q.m + sz : q.m - sz * (n2 - 1);
     q.hw = i > 0 || B.per[0];
     q.he = i < n0 - 1 || B.per[0];
     q.hs = j > 0 || B.per[1];
     q.hn = j < n1 - 1 || B.per[1];
     q.hb = k > 0 || B.per[2];
     q.ht = k < n2 - 1 || B.per[2];
+    // at a wall the cell itself (another cell of its colour may be being written)
+    const int wx = B.per[0] ? n0 - 1 : 0, wy = B.per[1] ? sy * (n1 - 1) : 0, wz = B.per[2] ? sz * (n2 - 1) : 0;
+    q.mw = q.m + (i > 0 ? -1 : wx);
+    q.me = q.m + (i < n0 - 1 ? 1 : -wx);
+    q.ms = q.m + (j > 0 ? -sy : wy);
+    q.mn = q.m + (j < n1 - 1 ? sy : -wy);
+    q.mb = q.m + (k > 0 ? -sz : wz);
+    q.mt = q.m + (k < n2 - 1 ? sz : -wz);
     return q;
 }
 
@@ -239,7 +289,10 @@ __device__ inline void cc_terms(const T* sm, const CcLvl& l, const CcNb& q, T& a
     a6 = sm[l.cz + q.m];
 }
 
-template <typename T>
+// SEAM: the coarsest level has a periodic axis with an odd extent (a kernel of
+// its own: in one, the further passes took registers from all, 58 to 117 us for the
+// FP64 cycle of 16^3 cells)
+template <typename T, bool SEAM>
 __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, int L0, int nl, const Bnd B, int nu1,
                                                             int nu2, int nuc, int cf, int ct, int scratch) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
@@ -292,8 +345,18 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
         if (warp) __syncwarp();
         else __syncthreads();
     };
+    auto update = [&](const CcLvl& l, T w, int i, int j, int k) {
+        const CcNb q = cc_nb(l, B, i, j, k);
+        T a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt;
+        cc_terms(sm, l, q, a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt);
+        T d = a1 + a2 + a3 + a4 + a5 + a6;
+        T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + sm[l.b + q.m];
+        T* x = sm + l.x;
+        if (d > (T)0) x[q.m] = relax(s / d, w != (T)1 ? x[q.m] : (T)0, w);
+    };
     // one colour pass of red-black Gauss-Seidel over level l
     auto smooth = [&](const CcLvl& l, T w, int color, bool warp) {
+        const int axes = SEAM ? seam_axes(B, l.n0, l.n1, l.n2) : 0;   // (none but on the coarsest)
         const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
         const int h0 = (l.n0 + 1) >> 1, hn = h0 * l.n1;
         const int tot = hn * l.n2;
@@ -302,16 +365,15 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
             const int k = div_small(t, hn, rhn), r = t - k * hn;
             const int j = div_small(r, h0, rh0), ih = r - j * h0;
             const int i = 2 * ih + ((j + k + color) & 1);
-            if (i >= l.n0) continue;
-            const CcNb q = cc_nb(l, B, i, j, k);
-            T a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt;
-            cc_terms(sm, l, q, a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt);
-            T d = a1 + a2 + a3 + a4 + a5 + a6;
-            T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + sm[l.b + q.m];
-            T* x = sm + l.x;
-            if (d > (T)0) x[q.m] = relax(s / d, w != (T)1 ? x[q.m] : (T)0, w);
+            if (i >= l.n0 || (SEAM && seam_count(B, l.n0, l.n1, l.n2, i, j, k))) continue;
+            update(l, w, i, j, k);
         }
         sync(warp);
+        for (int count = 1; count <= axes; count++) {
+            for_seam_cells(B, l.n0, l.n1, l.n2, color, count, t0, st,
+                           [&](int i, int j, int k) { update(l, w, i, j, k); });
+            sync(warp);
+        }
     };
     auto down = [&](int L, bool warp) {   // zero, pre-smooth and restrict level L, or solve the coarsest
         const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
@@ -1056,8 +1118,8 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_CUDA_TRY(c, cudaMemsetAsync(l.x, 0, l.N * sizeof(T), c->stream));
             LV<T> v = view(l);
             for (int s = 0; s < nu1; s++) {
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
             }
             cur[L] = l.x;
         }
@@ -1069,10 +1131,16 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
     if (lv[Lc].N > kCoarseCells) {   // the coarsest, too large for a block
         const LV<T> v = view(lv[Lc]);
         PARIS_CUDA_TRY(c, cudaMemsetAsync(v.x, 0, v.N * sizeof(T), c->stream));
+        const bool seam = seam_axes(c->bnd, v.n0, v.n1, v.n2) > 0;
+        const dim3 grid = row_grid((v.n0 + 1) / 2, v.n1, v.n2);
         for (int s = 0; s < 4 * kCoarseSweeps; s++) {
             const int color = s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1);
-            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2),
-                           128, 0, v, c->bnd, color);
+            if (seam) {
+                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, (k_fast_smooth<T, true>), grid, 128, 0, v, c->bnd, color);
+                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), 0L, k_fast_smooth_seam<T>, 1, 1024, 0, v, c->bnd, color);
+            } else {
+                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, (k_fast_smooth<T, false>), grid, 128, 0, v, c->bnd, color);
+            }
         }
     } else {
         LVSet<T> S;
@@ -1083,12 +1151,16 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
         const size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
         static size_t csm_set = 0;   // opt-in size set for this instantiation
         if (csm > csm_set) {
-            PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k_coarse_cycle_smem<T>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+            for (auto* k : {&k_coarse_cycle_smem<T, false>, &k_coarse_cycle_smem<T, true>})
+                PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
             csm_set = csm;
         }
-        PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, k_coarse_cycle_smem<T>, 1, 1024, csm, S, Lc, nl,
-                       c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
+        if (seam_axes(c->bnd, lv[nl - 1].n[0], lv[nl - 1].n[1], lv[nl - 1].n[2]))
+            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, (k_coarse_cycle_smem<T, true>), 1, 1024, csm, S,
+                           Lc, nl, c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
+        else
+            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, (k_coarse_cycle_smem<T, false>), 1, 1024, csm, S,
+                           Lc, nl, c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
     }
     cur[Lc] = lv[Lc].x;
     for (int L = Lc - 1; L >= 0; L--) {
@@ -1119,8 +1191,8 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_LAUNCH_N(c, kname<T>("mg_prolong"), v.N, k_fast_prolong<T>, row_grid(v.n0, v.n1, v.n2), 128, 0, v,
                            view_x(lv[L + 1], cur[L + 1]));
             for (int s = 0; s < nu2; s++) {
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
             }
         }
     }

@@ -1,7 +1,9 @@
 // The multigrid's smoothing kernels on the CPU (cuda_on_host.h) against the
 // colour passes written out; ThreadSanitizer ends the program at the first race.
-// Arguments: column sweep: "col <float|double> <configuration> n0 n1 n2 px py pz
-// form zc", form 0 plain, 1 zero iterate, 2 with the coarse correction.
+// Arguments: "col <float|double> <configuration> n0 n1 n2 px py pz form zc", the
+// column sweep, form 0 plain, 1 zero iterate, 2 with the coarse correction;
+// "coarse <type> <levels> n0 n1 n2 px py pz threads", the cycle in shared memory;
+// "passes <type> 0 n0 n1 n2 px py pz", colour passes by launches.
 static double rnd() {
     static uint64_t s = 88172645463325252ull;
     s ^= s << 13; s ^= s >> 7; s ^= s << 17;
@@ -92,10 +94,47 @@ static int run_col(const int* n, const int* per, int form, int zc) {
     return bad;
 }
 
+template <typename T>
+static int run_coarse(const int* n, const int* per, int nl, unsigned threads) {
+    LVSet<T> S{};
+    std::vector<Problem<T>*> p;
+    size_t cells = 0;
+    for (int L = 0; L < nl; L++) {
+        p.push_back(new Problem<T>(n[0] >> L, n[1] >> L, n[2] >> L, per));
+        S.l[L] = p[L]->view(p[L]->x, (T)1.1);
+        cells += 5 * S.l[L].N;
+    }
+    const LV<T>& last = S.l[nl - 1];
+    auto* const kernel = seam_axes(p[0]->B, last.n0, last.n1, last.n2) ? &k_coarse_cycle_smem<T, true> : &k_coarse_cycle_smem<T, false>;
+    launch(dim3(1), threads, [&] { kernel(S, 0, nl, p[0]->B, 2, 2, 0, 1, 0, (int)cells); });
+    if (nl > 1) return 0;   // (races only)
+    std::vector<T> ref(S.l[0].N, (T)0);
+    const LV<T> r = p[0]->view(ref.data(), (T)1.1);
+    for (int s = 0; s < 4 * kCoarseSweeps; s++) pass(r, p[0]->B, s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1), false);
+    return same(p[0]->x, ref.data(), r.N, "coarse cycle");
+}
+
+// colour passes over a whole level by launches, two passes
+template <typename T>
+static int run_passes(const int* n, const int* per) {
+    Problem<T> p(n[0], n[1], n[2], per);
+    const LV<T> v = p.view(p.x, (T)1.1);
+    std::vector<T> ref(p.x, p.x + v.N);
+    const LV<T> r = p.view(ref.data(), (T)1.1);
+    for (int color = 0; color < 2; color++) {
+        launch(dim3(1, n[1], n[2]), 32, [&] { k_fast_smooth<T, true>(v, p.B, color); });
+        launch(dim3(1), 64, [&] { k_fast_smooth_seam<T>(v, p.B, color); });
+        pass(r, p.B, color, false);
+    }
+    return same(p.x, ref.data(), v.N, "colour passes");
+}
+
 int main(int argc, char** argv) {
     auto arg = [&](int q) { return q < argc ? atoi(argv[q]) : 0; };
     const std::string kind = argv[1], type = argv[2];
     const int n[3] = {arg(4), arg(5), arg(6)}, per[3] = {arg(7), arg(8), arg(9)};
+    if (kind == "coarse") return type == "float" ? run_coarse<float>(n, per, arg(3), arg(10)) : run_coarse<double>(n, per, arg(3), arg(10));
+    if (kind == "passes") return type == "float" ? run_passes<float>(n, per) : run_passes<double>(n, per);
 #define COL(t, id, ...) \
     if (kind == "col" && type == #t && arg(3) == id) return run_col<SwColCfg<t, __VA_ARGS__>>(n, per, arg(10), arg(11));
     COLUMN_CONFIGURATIONS

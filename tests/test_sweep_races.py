@@ -74,3 +74,18 @@ def run(program, *args):
     (3, (32, 8, 6), (1, 1, 1), 4), (3, (20, 8, 6), (0, 0, 1), 2), (4, (60, 12, 4), (1, 0, 0), 4)])
 def test_column_sweep(program, cfg, n, per, zc, form):
     run(program, "col", CONFIGS[cfg][0], cfg, *n, *per, form, zc)
+
+
+# coarsest levels: odd extents over periodic seams (one, two, three axes), in a
+# block and in one warp, and the levels above them
+@pytest.mark.parametrize("ftype", ["float", "double"])
+@pytest.mark.parametrize("nl,n,per", [(1, (5, 4, 7), (1, 1, 0)), (1, (3, 9, 5), (1, 1, 1)), (1, (3, 3, 5), (1, 1, 1)),
+                                      (1, (6, 5, 4), (0, 1, 1)), (1, (5, 7, 3), (0, 0, 0)), (2, (6, 10, 6), (1, 1, 1))])
+def test_coarse_cycle(program, nl, n, per, ftype):
+    """One level: also the 32 passes cell after cell, to the bit."""
+    run(program, "coarse", ftype, nl, *n, *per, 64)
+
+
+@pytest.mark.parametrize("n,per", [((5, 7, 9), (1, 1, 1)), ((9, 4, 5), (1, 0, 1)), ((6, 5, 8), (1, 1, 1))])
+def test_colour_passes(program, n, per):
+    run(program, "passes", "double", 0, *n, *per)
