@@ -15,7 +15,18 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 ORACLE_RTOL = 1e-8     # GPU adjoint vs oracle adjoint (both FP64, solves to 1e-12 / 1e-15)
-FD_RTOL = 1e-6         # adjoint vs central differences, eps = 1e-6 (relative for rho), per entry
+FD_RTOL = 1e-6         # adjoint vs central differences, per entry
+# Step of the central differences (relative for rho).  Two forwards differ by the
+# rounding of their pressures and velocities, whatever the step, so the quotient
+# carries an error of 1.6e-13 / eps (rms over the entries; 1.7e-7, 1.6e-8 and
+# 1.6e-9 measured at 1e-6, 1e-5 and 1e-4).  The bound of the rounding of the
+# stored pressure alone is sqrt(sum over cells of (dL/dp ulp(p))^2 / 12) =
+# 8.5e-14 for each rounding and forward, 0.85e-13 / eps for the two that end a
+# solve.  Entries are checked from a fifth of the largest (1.5) up: three
+# times that rms over 0.3 is 1.6e-6 at a step of 1e-6, above FD_RTOL whatever the
+# gradient is worth, and 1.6e-7 at 1e-5.  u* enters linearly and the truncation in
+# rho goes as eps^2: no part of the 1e-9 left at 1e-4.
+FD_EPS = 1e-5
 FD_FLOOR = 0.2         # entries checked per entry: |gradient| >= FD_FLOOR * the largest sampled one
 
 
@@ -95,7 +106,7 @@ def fd_forward(gpu, capi, dt, us, p0):
     """A forward for differencing, from the unperturbed pressure: FP64 PCG to
     ||r||/||b|| < 1e-15, then four FP64 defect-correction cycles that take the
     true residual b - A p to its FP64 floor (the base solve's 1e-14 would
-    leave ~1e-5 of the response to a 1e-6 perturbation unresolved at 128^3;
+    leave ~1e-6 of the response to a 1e-5 perturbation unresolved at 128^3;
     CG itself is not run below the floor, where its recurrences drift)."""
     gpu_forward(gpu, capi, dt, us, p0, rel_tol=1e-15, maxit=60, project=False)
     with warnings.catch_warnings():
@@ -127,7 +138,7 @@ def test_adjoint_finite_differences_128(gpu_lib, capi, runtime, orc):
         for _ in range(120):
             k = int(rng.integers(3))
             q = tuple(int(rng.integers(g, g + n)) for _ in range(3))
-            eps = 1e-6
+            eps = FD_EPS
             up = [a.copy() for a in us]
             up[k][q] += eps
             orc.fill_ghosts(d, up[k])
@@ -142,7 +153,7 @@ def test_adjoint_finite_differences_128(gpu_lib, capi, runtime, orc):
         for _ in range(80):
             q = tuple(int(rng.integers(0, n)) for _ in range(3))
             qq = tuple(c + g for c in q)
-            eps = 1e-6 * rho[qq]
+            eps = FD_EPS * rho[qq]
             res = []
             for s in (1.0, -1.0):
                 r1 = rho.copy()
@@ -165,8 +176,8 @@ def test_adjoint_finite_differences_128(gpu_lib, capi, runtime, orc):
               f"{rel.max():.3e} median {np.median(rel):.3e}; below the floor max |fd-ad|/max|ad| {absl:.3e}")
         assert big.sum() >= len(e) // 3, name
         assert rel.max() < FD_RTOL, name
-        # the absolute error of the central differences, measured 1.1e-7 (u*)
-        # and 2.7e-7 (rho) of the largest gradient
+        # the absolute error of the central differences, measured 1.3e-8 (u*)
+        # and 2.5e-8 (rho) of the largest gradient
         assert absl < 5e-7, name
     assert np.abs(np.concatenate([a.ravel() for a in u0])).max() > 0
 
