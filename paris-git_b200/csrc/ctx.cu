@@ -92,6 +92,31 @@ int ctx_ghost_fill_i8(paris_ctx* c, int8_t* f) {
     return PARIS_OK;
 }
 
+int ctx_kernel_blocks(paris_ctx* c, const void* kernel, int threads, size_t smem) {
+    for (const auto& u : c->kernels)
+        if (u.kernel == kernel && u.smem >= smem) return u.per_sm;
+    int per = 0;
+    cudaError_t e = cudaSuccess;
+    if (smem > 0) {
+        // all that the device gives: another handle may need more than this one
+        int most = 0;
+        cudaFuncAttributes f{};
+        e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&f, kernel);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)f.sharedSizeBytes);
+    }
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
+    if (e != cudaSuccess || per < 1) {
+        cudaGetLastError();
+        ctx_set_error(c, "a kernel of %d threads and %zu bytes of shared memory cannot run: %s", threads, smem,
+                      cudaGetErrorString(e));
+        return 0;
+    }
+    c->kernels.push_back({kernel, smem, per});
+    return per;
+}
+
 // ---- reductions -----------------------------------------------------------
 // Kernels write kRedBlocks partials per slot; this sums them in a fixed order.
 __global__ void k_reduce_slots(const double* __restrict__ part, double* out, int op_max, int nb) {

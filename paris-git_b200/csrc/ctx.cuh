@@ -77,7 +77,12 @@ struct paris_ctx {
     double* red_host_dev = nullptr;   // its device address
     int red_nb = kRedBlocks;       // blocks of the last reduction launch
     int nsm = 148;
-    std::vector<std::pair<const void*, int>> red_occ;   // kernel -> resident blocks per SM
+    struct KernelUse {
+        const void* kernel;
+        size_t smem;
+        int per_sm;
+    };
+    std::vector<KernelUse> kernels;   // ctx_kernel_blocks
     // multigrid hierarchies
     int ref_lmg = 0;
     std::vector<RefLevel> ref;     // index 1..LMG
@@ -124,18 +129,19 @@ struct paris_ctx {
 };
 
 
+// Resident blocks per SM of a kernel with smem bytes of dynamic shared memory
+// (0: the device refuses it; the error is set).  Lifts the kernel's limit of
+// 48 KB on first use: it belongs to the kernel on one device, and a process may
+// drive handles of several devices from several threads, so each handle keeps
+// its own record.
+int ctx_kernel_blocks(paris_ctx* c, const void* kernel, int threads, size_t smem);
+
 // Grid of a reduction kernel: one wave of resident blocks (at most
 // kRedBlocks); records the block count for ctx_reduce_finish.
 template <typename K>
 unsigned red_grid(paris_ctx* c, K kernel, int threads) {
-    const void* key = (const void*)kernel;
-    int per = 0;
-    for (auto& e : c->red_occ)
-        if (e.first == key) per = e.second;
-    if (!per) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0) != cudaSuccess || per < 1) per = 1;
-        c->red_occ.push_back({key, per});
-    }
+    int per = ctx_kernel_blocks(c, (const void*)kernel, threads, 0);
+    if (per < 1) per = 1;
     int g = per * c->nsm;
     if (g > kRedBlocks) g = kRedBlocks;
     c->red_nb = g;

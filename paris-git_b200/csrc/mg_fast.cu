@@ -723,19 +723,13 @@ using TmEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to
 // the driver library); null when the driver does not provide it
 static TmEncodeFn tm_encode_fn() {
-    static TmEncodeFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (TmEncodeFn)p;
-        else
-            cudaGetLastError();
-    }
-    return fn;
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+        return (TmEncodeFn)p;
+    cudaGetLastError();
+    return nullptr;
 }
 
 // a level array as the 3-D tensor (n0, n1, n2), boxes of a tile and its ring;
@@ -862,13 +856,7 @@ static int fast_coefs(paris_ctx* c) {
 template <class Cfg>
 static int sweep_merged_chunk(paris_ctx* c, const FastLevel<float>& l) {
     constexpr size_t smem = sweep2_smem_cfg<Cfg>();
-    static int per_sm = 0;   // resident blocks per SM (the same on every B200)
-    if (!per_sm) {
-        cudaFuncSetAttribute(k_rb_sweep2_cfg<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep2_cfg<Cfg>, Cfg::NT, smem) !=
-                cudaSuccess || per_sm < 1)
-            per_sm = 1;
-    }
+    const int per_sm = ctx_kernel_blocks(c, (const void*)k_rb_sweep2_cfg<Cfg>, Cfg::NT, smem);
     long tiles = (long)div_up(l.n[0], Cfg::TX) * div_up(l.n[1], Cfg::TY);
     long nbz = (long)per_sm * c->nsm / tiles;
     long cap = l.n[2] / 4;
@@ -893,17 +881,10 @@ static int sweep_merged(paris_ctx* c, const FastLevel<float>& l, const char* lab
     return PARIS_OK;
 }
 
-// planes per block of the TMA-staged sweep, as sweep_chunk
+// planes per block of the TMA-staged sweep, as sweep_merged_chunk
 static int sweep_tma_chunk(paris_ctx* c, const FastLevel<float>& l) {
     using Cfg = SwTmaCfg;
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaFuncSetAttribute(k_rb_sweep_tma<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sweep_tma_smem<Cfg>());
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep_tma<Cfg>, Cfg::NT,
-                                                          sweep_tma_smem<Cfg>()) != cudaSuccess || per_sm < 1)
-            per_sm = 1;
-    }
+    const int per_sm = ctx_kernel_blocks(c, (const void*)k_rb_sweep_tma<Cfg>, Cfg::NT, sweep_tma_smem<Cfg>());
     long tiles = (long)div_up(l.n[0], Cfg::TX) * div_up(l.n[1], Cfg::TY);
     long nbz = (long)per_sm * c->nsm / tiles;
     long cap = l.n[2] / 4;
@@ -939,16 +920,11 @@ template <class C, bool ZERO, bool CORR>
 static int sweep_col_launch(paris_ctx* c, const char* label, const FastLevel<typename C::T>& l,
                             const typename C::T* xin, typename C::T* xout, const typename C::T* xc, int first,
                             double* bx_part, int* bx_blocks) {
-    static bool set = false;   // (the same value by every thread)
-    if (!set) {
-        PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k_rb_sweep_col<C, ZERO, CORR>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-        set = true;
-    }
+    auto* const kern = &k_rb_sweep_col<C, ZERO, CORR>;
+    if (!ctx_kernel_blocks(c, (const void*)kern, C::NT, C::SMEM)) return PARIS_CUDA_ERROR;
     const SwColGeo g = sweep_col_geo<C>(c, l);
     const dim3 grid(div_up(l.n[0], g.W), div_up(l.n[1], C::TY), div_up(l.n[2], g.zc));
     if (bx_part && (long)grid.x * grid.y * grid.z > kRedBlocks) bx_part = nullptr;
-    auto* const kern = &k_rb_sweep_col<C, ZERO, CORR>;
     PARIS_LAUNCH_N(c, label, l.N, kern, grid, C::NT, C::SMEM, view(l), xin, xout, xc, c->bnd, first, g, bx_part);
     if (bx_part && bx_blocks) *bx_blocks = (int)(grid.x * grid.y * grid.z);
     return PARIS_OK;
@@ -1011,14 +987,7 @@ static int sweep_fused(paris_ctx* c, int L, const FastLevel<T>& l, const T* xin,
 // blocks, an even number of planes, at least 4
 static int sweep_rs_chunk(paris_ctx* c, const FastLevel<float>& l) {
     using Cfg = SwRsCfg;
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaFuncSetAttribute(k_rb_sweep_rs<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sweep_rs_smem<Cfg>());
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep_rs<Cfg>, Cfg::NT,
-                                                          sweep_rs_smem<Cfg>()) != cudaSuccess || per_sm < 1)
-            per_sm = 1;
-    }
+    const int per_sm = ctx_kernel_blocks(c, (const void*)k_rb_sweep_rs<Cfg>, Cfg::NT, sweep_rs_smem<Cfg>());
     long tiles = (long)div_up(l.n[0], Cfg::TX) * div_up(l.n[1], Cfg::TY);
     long nbz = (long)per_sm * c->nsm / tiles;
     long cap = l.n[2] / 4;
@@ -1040,19 +1009,12 @@ static int sweep_rs(paris_ctx* c, const FastLevel<float>& l, const FastLevel<flo
     return PARIS_OK;
 }
 
-// planes per block of the pair sweep: as sweep_chunk, at least 8 planes per
+// planes per block of the pair sweep: as sweep_merged_chunk, at least 8 planes per
 // block (a block recomputes three planes on either side of its chunk)
 template <typename T>
 static int sweep4_chunk(paris_ctx* c, const FastLevel<T>& l) {
     using Cfg = typename SwGeo4<T>::Cfg;
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaFuncSetAttribute(k_rb_sweep4_cfg<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sweep4_smem_cfg<Cfg>());
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rb_sweep4_cfg<Cfg>, Cfg::NT,
-                                                          sweep4_smem_cfg<Cfg>()) != cudaSuccess || per_sm < 1)
-            per_sm = 1;
-    }
+    const int per_sm = ctx_kernel_blocks(c, (const void*)k_rb_sweep4_cfg<Cfg>, Cfg::NT, sweep4_smem_cfg<Cfg>());
     long tiles = (long)div_up(l.n[0], Cfg::TX) * div_up(l.n[1], Cfg::TY);
     long nbz = (long)per_sm * c->nsm / tiles;
     long cap = l.n[2] / 8;
@@ -1149,18 +1111,12 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
         // shared memory (at most 219 KB, FP64 from 16^3 down)
         const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
         const size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
-        static size_t csm_set = 0;   // opt-in size set for this instantiation
-        if (csm > csm_set) {
-            for (auto* k : {&k_coarse_cycle_smem<T, false>, &k_coarse_cycle_smem<T, true>})
-                PARIS_CUDA_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-            csm_set = csm;
-        }
-        if (seam_axes(c->bnd, lv[nl - 1].n[0], lv[nl - 1].n[1], lv[nl - 1].n[2]))
-            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, (k_coarse_cycle_smem<T, true>), 1, 1024, csm, S,
-                           Lc, nl, c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
-        else
-            PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, (k_coarse_cycle_smem<T, false>), 1, 1024, csm, S,
-                           Lc, nl, c->bnd, nu1_, nu2_, nuc, cf, ct, (int)scratch);
+        const FastLevel<T>& last = lv[nl - 1];
+        auto* const kern = seam_axes(c->bnd, last.n[0], last.n[1], last.n[2]) ? &k_coarse_cycle_smem<T, true>
+                                                                              : &k_coarse_cycle_smem<T, false>;
+        if (!ctx_kernel_blocks(c, (const void*)kern, 1024, csm)) return PARIS_CUDA_ERROR;
+        PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, kern, 1, 1024, csm, S, Lc, nl, c->bnd, nu1_, nu2_, nuc,
+                       cf, ct, (int)scratch);
     }
     cur[Lc] = lv[Lc].x;
     for (int L = Lc - 1; L >= 0; L--) {
