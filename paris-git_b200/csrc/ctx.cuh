@@ -18,6 +18,13 @@ struct RefLevel {
     double* q;   // beta / K7
 };
 
+// Geometry of a launch of the column sweep: W output cells across a tile, H ring
+// cells on either side (0: the tile is the whole row), lanes = (W + 2 H) / VEC
+// chunks in use, zc planes per block (even)
+struct SwColGeo {
+    int W, H, lanes, zc;
+};
+
 // One level of the B200 multigrid: face coefficients (east/north/top of each
 // cell) and work vectors, in T = float (inner cycle of the mixed solver) and
 // double (the FP64 solver).
@@ -32,6 +39,8 @@ struct FastLevel {
     bool pairs = false;    // two consecutive sweeps run as one pass (k_rb_sweep4_cfg)
     bool rs = false;       // the last pre-smoothing sweep forms the coarse right-hand side (k_rb_sweep_rs)
     int merged = 0;        // FP32: the fused sweep with one barrier per step (1: 32x12 tiles, 2: 32x14)
+    int col_cfg = 0;       // the column sweep's configuration and launch geometry on this level
+    SwColGeo col{};
     double omega = 1.0;    // relaxation factor of the red-black smoother, set by each solve
 };
 

@@ -809,6 +809,65 @@ void mg_fast_free_maps(paris_ctx* c) {
     }
 }
 
+// The configurations of the column sweep: f(SwColCfg<...>{}) of number cfg.
+template <typename T, typename F>
+static int with_col_cfg(int cfg, F f) {
+    constexpr bool s = sizeof(T) == 4;
+    switch (cfg) {
+        case 0: return f(SwColCfg<T, 16, 6, s ? 3 : 2, 4>{});
+        case 1: return f(SwColCfg<T, 32, s ? 6 : 4, 2, s ? 2 : 3>{});
+        case 2: return f(SwColCfg<T, 48, s ? 5 : 8, s ? 1 : 2, s ? 2 : 1>{});
+        case 3: return f(SwColCfg<T, 64, s ? 7 : 8, 2, 1>{});
+        case 4: return f(SwColCfg<T, 16, 10, 2, 3>{});
+        default: break;
+    }
+    if constexpr (s) return f(SwColCfg<T, 128, 4, 1, 1>{});
+    return PARIS_BAD_ARGS;
+}
+
+// Launch geometry of the column sweep with configuration C on level l: planes
+// per block (even) so that the blocks fill whole waves of the C::MINB x nsm
+// resident ones with long chunks (a chunk takes about three planes' time before
+// its first output).
+template <class C>
+static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l) {
+    const int n0 = l.n[0], n2 = l.n[2];
+    SwColGeo g;
+    sweep_col_tiles<C>(n0, g);
+    const long tiles = (long)div_up(n0, g.W) * div_up(l.n[1], C::TY), slots = (long)C::MINB * c->nsm;
+    double best = -1.0;
+    g.zc = n2;
+    for (int zc = 2; zc <= n2; zc += 2) {
+        const long blocks = tiles * div_up(n2, zc), waves = (blocks + slots - 1) / slots;
+        const double eff = (double)tiles * n2 / (double)(waves * slots * (zc + 3));
+        if (eff > best) {
+            best = eff;
+            g.zc = zc;
+        }
+    }
+    return g;
+}
+
+// Configuration and geometry of the column sweep on a level, once per handle.
+// Rows of up to 64 chunks, and (FP32) of 97 to 128, as whole rows: no ring
+// columns, and a warp's lanes lie in rows of one parity.  Other rows are cut
+// into tiles of up to 14 output chunks.
+// Measured us per sweep (B200), this form / the two-phase form it replaced:
+// FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 184x180x100 30 / 38, 256^3 84 / 138,
+// 512x256x128 106 / 138, 320x192x160 (cut) 70 / 89; FP64 64^3 9.8 / 10.8,
+// 96x64x80 13.3 / 15.3, 128^3 30 / 44, 144x176x56 (cut) 28 / 38, 256x128x128
+// (cut) 69 / 78, 208x112x32 (cut) 19.5 / 19.2.
+template <typename T>
+static int sweep_col_choose(const paris_ctx* c, FastLevel<T>& l) {
+    const int chunks = l.n[0] * (int)sizeof(T) / 16;
+    l.col_cfg = chunks <= 16 ? 0 : (chunks <= 32 ? 1 : (chunks <= 48 ? 2 : (chunks <= 64 ? 3 : 4)));
+    if (sizeof(T) == 4 && chunks > 96 && chunks <= 128) l.col_cfg = 5;
+    return with_col_cfg<T>(l.col_cfg, [&](auto cfg) {
+        l.col = sweep_col_geo<decltype(cfg)>(c, l);
+        return (int)PARIS_OK;
+    });
+}
+
 template <typename T>
 static int fast_alloc(paris_ctx* c) {
     auto& lv = levels<T>(c);
@@ -825,7 +884,10 @@ static int fast_alloc(paris_ctx* c) {
         l.x2 = nullptr;
         bool fusable = l.N >= kFusedCells && l.N > kCoarseCells && l.n[0] % 4 == 0 && l.n[1] % 2 == 0 &&
                        l.n[2] % 2 == 0 && L < nl - 1 && l.N < 1L << 32;
-        if (fusable) PARIS_CUDA_TRY(c, cudaMalloc(&l.x2, l.N * sizeof(T)));
+        if (fusable) {
+            PARIS_CUDA_TRY(c, cudaMalloc(&l.x2, l.N * sizeof(T)));
+            PARIS_CHECK(sweep_col_choose(c, l));
+        }
         l.pairs = fusable && pairs_wanted();
         l.rs = fusable && std::is_same<T, float>::value && (rs_levels() == 2 || (rs_levels() == 1 && L == 0));
         l.merged = fusable && std::is_same<T, float>::value ? merged_wanted() : 0;
@@ -893,49 +955,18 @@ static int sweep_tma_chunk(paris_ctx* c, const FastLevel<float>& l) {
     return (int)div_up(l.n[2], nbz);
 }
 
-// Launch geometry of the column sweep with configuration C on level l: planes
-// per block (even) so that the blocks fill whole waves of the C::MINB x nsm
-// resident ones with long chunks (a chunk takes about three planes' time before
-// its first output).
-template <class C>
-static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l) {
-    const int n0 = l.n[0], n2 = l.n[2];
-    SwColGeo g;
-    sweep_col_tiles<C>(n0, g);
-    const long tiles = (long)div_up(n0, g.W) * div_up(l.n[1], C::TY), slots = (long)C::MINB * c->nsm;
-    double best = -1.0;
-    g.zc = n2;
-    for (int zc = 2; zc <= n2; zc += 2) {
-        const long blocks = tiles * div_up(n2, zc), waves = (blocks + slots - 1) / slots;
-        const double eff = (double)tiles * n2 / (double)(waves * slots * (zc + 3));
-        if (eff > best) {
-            best = eff;
-            g.zc = zc;
-        }
-    }
-    return g;
-}
-
 template <class C, bool ZERO, bool CORR>
 static int sweep_col_launch(paris_ctx* c, const char* label, const FastLevel<typename C::T>& l,
                             const typename C::T* xin, typename C::T* xout, const typename C::T* xc, int first,
                             double* bx_part, int* bx_blocks) {
     auto* const kern = &k_rb_sweep_col<C, ZERO, CORR>;
     if (!ctx_kernel_blocks(c, (const void*)kern, C::NT, C::SMEM)) return PARIS_CUDA_ERROR;
-    const SwColGeo g = sweep_col_geo<C>(c, l);
+    const SwColGeo g = l.col;
     const dim3 grid(div_up(l.n[0], g.W), div_up(l.n[1], C::TY), div_up(l.n[2], g.zc));
     if (bx_part && (long)grid.x * grid.y * grid.z > kRedBlocks) bx_part = nullptr;
     PARIS_LAUNCH_N(c, label, l.N, kern, grid, C::NT, C::SMEM, view(l), xin, xout, xc, c->bnd, first, g, bx_part);
     if (bx_part && bx_blocks) *bx_blocks = (int)(grid.x * grid.y * grid.z);
     return PARIS_OK;
-}
-
-template <class C>
-static int sweep_col(paris_ctx* c, const char* label, const FastLevel<typename C::T>& l, const typename C::T* xin,
-                     typename C::T* xout, const typename C::T* xc, int first, double* bx_part, int* bx_blocks) {
-    if (!xin) return sweep_col_launch<C, true, false>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
-    if (xc) return sweep_col_launch<C, false, true>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
-    return sweep_col_launch<C, false, false>(c, label, l, xin, xout, xc, first, bx_part, bx_blocks);
 }
 
 // bx_part: also write the per-block partials of b.x (see k_rb_sweep_col);
@@ -961,26 +992,13 @@ static int sweep_fused(paris_ctx* c, int L, const FastLevel<T>& l, const T* xin,
         if (l.merged == 1) return sweep_merged<SwMCfg12>(c, l, label, xin, xout, xc, first, bx_part, bx_blocks);
         if (l.merged == 2) return sweep_merged<SwMCfg14>(c, l, label, xin, xout, xc, first, bx_part, bx_blocks);
     }
-    const int chunks = l.n[0] * (int)sizeof(T) / 16;
     const char* name = kname<T>(label);
-#define SWEEP_COL(P, TY, D, MINB) \
-    return sweep_col<SwColCfg<T, P, TY, D, MINB>>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks)
-    // Rows of up to 64 chunks, and (FP32) of 97 to 128, as whole rows: no ring
-    // columns, and a warp's lanes lie in rows of one parity.  Other rows are cut
-    // into tiles of up to 14 output chunks.
-    // Measured us per sweep (B200), this form / the two-phase form it replaced:
-    // FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 184x180x100 30 / 38, 256^3 87 / 138,
-    // 512x256x128 114 / 138, 320x192x160 (cut) 72 / 89; FP64 64^3 9.8 / 10.8,
-    // 96x64x80 13.3 / 15.3, 128^3 30 / 44, 144x176x56 (cut) 28 / 38, 256x128x128
-    // (cut) 69 / 78, 208x112x32 (cut) 19.5 / 19.2.
-    if (chunks <= 16) SWEEP_COL(16, 6, sizeof(T) == 4 ? 3 : 2, 4);
-    if (chunks <= 32) SWEEP_COL(32, (sizeof(T) == 4 ? 6 : 4), 2, (sizeof(T) == 4 ? 2 : 3));
-    if (chunks <= 48) SWEEP_COL(48, (sizeof(T) == 4 ? 5 : 8), (sizeof(T) == 4 ? 1 : 2), (sizeof(T) == 4 ? 2 : 1));
-    if (chunks <= 64) SWEEP_COL(64, (sizeof(T) == 4 ? 7 : 8), 2, 1);
-    if constexpr (sizeof(T) == 4)
-        if (chunks > 96 && chunks <= 128) SWEEP_COL(128, 4, 1, 1);
-    SWEEP_COL(16, 10, 2, 3);
-#undef SWEEP_COL
+    return with_col_cfg<T>(l.col_cfg, [&](auto cfg) {
+        using C = decltype(cfg);
+        if (!xin) return sweep_col_launch<C, true, false>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks);
+        if (xc) return sweep_col_launch<C, false, true>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks);
+        return sweep_col_launch<C, false, false>(c, name, l, xin, xout, xc, first, bx_part, bx_blocks);
+    });
 }
 
 // planes per block of the fused-restriction sweep: one wave of resident

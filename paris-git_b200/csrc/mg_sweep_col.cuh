@@ -74,13 +74,6 @@ struct alignas(16) SwChunk {
     T v[VEC];
 };
 
-// geometry of a launch: W output cells across a tile, H ring cells on either
-// side (0: the tile is the whole row), lanes = (W + 2 H) / VEC <= PITCH chunks
-// in use, zc planes per block (even)
-struct SwColGeo {
-    int W, H, lanes, zc;
-};
-
 // the tiles across a row of n0 cells: as wide as the grid where its chunks fit
 // a staged row, else equal tiles with one ring chunk on either side
 template <class C>

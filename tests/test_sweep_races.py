@@ -31,7 +31,8 @@ def program(tmp_path_factory):
     if not shutil.which("g++"):
         pytest.skip("no g++")
     read = lambda f: open(os.path.join(CSRC, f)).read()
-    fast, sweep, col, common = (read(f) for f in ("mg_fast.cu", "mg_sweep.cuh", "mg_sweep_col.cuh", "common.cuh"))
+    fast, sweep, col, common, ctx = (read(f) for f in ("mg_fast.cu", "mg_sweep.cuh", "mg_sweep_col.cuh", "common.cuh",
+                                                       "ctx.cuh"))
     col = col[:col.index("// 16 bytes, asynchronously")] + col[col.index("// a configuration:"):]
     text = "\n".join([
         between(common, "// Boundary description", "// The inflow of a 'jet'"),
@@ -39,6 +40,7 @@ def program(tmp_path_factory):
         "template <int BLOCK> double block_sum(double v, double*) { abort(); return v; }",
         between(fast, "static constexpr long kCoarseCells", "static inline dim3 row_grid"),
         between(sweep, "// wrap a coordinate into", "__device__ inline int sw_next"),
+        between(ctx, "struct SwColGeo", "// One level of the B200 multigrid"),
         col,
         between(fast, "// t / d for 0 <= t", "// shared memory of k_coarse_cycle_smem"),
     ])
