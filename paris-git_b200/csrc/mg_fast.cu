@@ -821,16 +821,19 @@ static int with_col_cfg(int cfg, F f) {
         case 4: return f(SwColCfg<T, 16, 10, 2, 3>{});
         default: break;
     }
-    if constexpr (s) return f(SwColCfg<T, 128, 4, 1, 1>{});
+    if constexpr (s) return cfg == 5 ? f(SwColCfg<T, 128, 4, 1, 1>{}) : f(SwColCfg<T, 48, 4, 1, 2>{});
     return PARIS_BAD_ARGS;
 }
 
 // Launch geometry of the column sweep with configuration C on level l: planes
 // per block (even) so that the blocks fill whole waves of the C::MINB x nsm
 // resident ones with long chunks (a chunk takes about three planes' time before
-// its first output).
+// its first output).  *cost: an estimate of the sweep's time that compares
+// configurations, the steps of each wave (planes per block + 3) times the time
+// of a step: a latency worth 24 warps' issue, and the warps resident on the
+// busiest SM; a tenth more for tiles, whose ring columns are loaded twice.
 template <class C>
-static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l) {
+static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>& l, double* cost) {
     const int n0 = l.n[0], n2 = l.n[2];
     SwColGeo g;
     sweep_col_tiles<C>(n0, g);
@@ -845,27 +848,43 @@ static SwColGeo sweep_col_geo(const paris_ctx* c, const FastLevel<typename C::T>
             g.zc = zc;
         }
     }
+    const long blocks = tiles * div_up(n2, g.zc), full = blocks / slots, rest = blocks % slots, warps = C::NT / 32;
+    double t = (double)full * (24 + C::MINB * warps);
+    if (rest) t += (double)(24 + ((rest + c->nsm - 1) / c->nsm) * warps);
+    *cost = t * (g.zc + 3) * (g.H ? 1.1 : 1.0);
     return g;
 }
 
-// Configuration and geometry of the column sweep on a level, once per handle.
-// Rows of up to 64 chunks, and (FP32) of 97 to 128, as whole rows: no ring
-// columns, and a warp's lanes lie in rows of one parity.  Other rows are cut
-// into tiles of up to 14 output chunks.
-// Measured us per sweep (B200), this form / the two-phase form it replaced:
-// FP32 64^3 8.2 / 9.1, 128^3 17.7 / 23.5, 184x180x100 30 / 38, 256^3 84 / 138,
-// 512x256x128 106 / 138, 320x192x160 (cut) 70 / 89; FP64 64^3 9.8 / 10.8,
-// 96x64x80 13.3 / 15.3, 128^3 30 / 44, 144x176x56 (cut) 28 / 38, 256x128x128
-// (cut) 69 / 78, 208x112x32 (cut) 19.5 / 19.2.
+// Configuration and geometry of the column sweep on a level, once per handle:
+// the cheapest by the estimate above, the first of equals.  Whole rows (no ring
+// columns, a warp's lanes in rows of one parity) win on large levels; on small
+// ones, where a wave is not full, many narrow blocks do.
+// Over 24 levels (FP32 and FP64, 48^3 to 320x192x160) the choice is within 0.3% of
+// the fastest configuration on average and 4% at most; by the row's length alone
+// (16, 32, 48, 64 chunks, else tiles) it was 2.9% and 15%.  Measured us per sweep
+// (B200, with the event's own 2 us), this choice / by length / the two-phase form
+// before: FP64 104x56x16 10.7 / 12.7 / 10.7, 160x96x48 18.9 / 21.0 / 22.1,
+// 208x112x32 21.9 / 21.9 / 20.9, 256x128x128 72.9 / 75.1 / 78.4; FP32 108x20x36
+// 9.5 / 10.7 / 9.2, 100x80x60 13.0 / 14.2 / 13.8, 216x40x72 14.4 / 14.8 / 14.7,
+// 176x96x48 14.7 / 15.9 / 15.0, 184x180x100 30.6 / 30.6 / 35.1.  Whole solves from
+// zero, us, this choice / by length / two-phase: FP64 208x112x32 2666 / 2779 / 2687,
+// 160x96x48 2924 / 3039 / 3116; FP32 176x96x48 2586 / 2660 / 2585, 216x40x72 3200 /
+// 3350 / 3295.
 template <typename T>
 static int sweep_col_choose(const paris_ctx* c, FastLevel<T>& l) {
-    const int chunks = l.n[0] * (int)sizeof(T) / 16;
-    l.col_cfg = chunks <= 16 ? 0 : (chunks <= 32 ? 1 : (chunks <= 48 ? 2 : (chunks <= 64 ? 3 : 4)));
-    if (sizeof(T) == 4 && chunks > 96 && chunks <= 128) l.col_cfg = 5;
-    return with_col_cfg<T>(l.col_cfg, [&](auto cfg) {
-        l.col = sweep_col_geo<decltype(cfg)>(c, l);
-        return (int)PARIS_OK;
-    });
+    double best = 0.0;
+    for (int cfg = 0; cfg < (sizeof(T) == 4 ? 7 : 5); cfg++)
+        PARIS_CHECK(with_col_cfg<T>(cfg, [&](auto t) {
+            double cost;
+            const SwColGeo g = sweep_col_geo<decltype(t)>(c, l, &cost);
+            if (cfg == 0 || cost < best) {
+                best = cost;
+                l.col_cfg = cfg;
+                l.col = g;
+            }
+            return (int)PARIS_OK;
+        }));
+    return PARIS_OK;
 }
 
 template <typename T>
