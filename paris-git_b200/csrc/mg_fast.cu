@@ -8,8 +8,9 @@
 //   the colours reversed after the coarse correction (symmetric cycle).
 // The inner cycle runs in T = float (mixed) or double; the outer loop is FP64:
 // defect correction p += V(b - A p), or CG preconditioned by the V-cycle.
-// Levels at or below kCoarseCells cells run in one single-block kernel; a
-// coarsest level above that is relaxed by the colour passes.
+// Levels at or below kCoarseCells cells run in one single-block kernel, as does
+// a larger coarsest level that fits its shared memory; above, the coarsest level
+// is relaxed by the colour passes.
 #include <stdlib.h>
 #include <string.h>
 #include <type_traits>
@@ -453,6 +454,15 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
         for (int t = tid; t < l.N; t += nt) g.x[t] = sm[l.x + t];
     }
 }
+
+// A coarsest level of more than 16^3 cells still runs in one block where its
+// five arrays fit (11.5 thousand cells FP32, 5.7 FP64), and by launches of colour
+// passes above.  Measured us per V-cycle (of grids four times as wide), one block
+// against launches, coarsest level of 17^3 cells 201 / 263 FP32 and 240 / 273
+// FP64, 25x20x15 229 / 265 FP32, 27x21x15 242 / 267 FP32; one block on global
+// memory, which larger ones took before, 346 / 293 at 33x25x15 FP32, 324 / 284 at
+// 25x20x15 FP64 and 6126 / 1326 at 95x65x55 FP32.
+static constexpr size_t kBlockSmem = 227 * 1024 - 1024;   // less the kernel's own
 
 // shared memory of k_coarse_cycle_smem: five arrays per level from L0 down
 template <typename T>
@@ -1127,7 +1137,7 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_LAUNCH_N(c, kname<T>("mg_restrict"), l.N, k_fast_restrict2<T>,
                            dim3(div_up(cv.n0, 32), cv.n1, cv.n2), dim3(32, 4), 0, view_x(l, cur[L]), cv, c->bnd);
     }
-    if (lv[Lc].N > kCoarseCells) {   // the coarsest, too large for a block
+    if (coarse_smem(lv, Lc) > kBlockSmem) {   // the coarsest, too large for a block
         const LV<T> v = view(lv[Lc]);
         PARIS_CUDA_TRY(c, cudaMemsetAsync(v.x, 0, v.N * sizeof(T), c->stream));
         const bool seam = seam_axes(c->bnd, v.n0, v.n1, v.n2) > 0;
@@ -1144,8 +1154,8 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
     } else {
         LVSet<T> S;
         for (int L = 0; L < nl; L++) S.l[L] = view(lv[L]);
-        // the levels and a scratch array of the largest restricted one fit the
-        // shared memory (at most 219 KB, FP64 from 16^3 down)
+        // from 16^3 down, the levels and a scratch array of the largest restricted
+        // one fit the shared memory (at most 219 KB, FP64)
         const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
         const size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
         const FastLevel<T>& last = lv[nl - 1];
