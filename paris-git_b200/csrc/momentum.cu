@@ -30,13 +30,16 @@ struct Vel {
 
 // The coordinate part of inter() for one face: xi and k from x0, x1, x2, x,
 // computed once per index on the host with the same IEEE operations (so the
-// values are those inter() forms), plus the reciprocals of k, 1 - k, k - 1.
-// On a uniform grid with a power-of-two cell count k = -1, so the divisions
-// of inter() by k, 1 - k and k - 1 are by powers of two: multiplying by the
-// exact reciprocal then rounds to the same double as dividing, and the
-// kernel takes that form (R = true) when every reciprocal it uses is exact.
+// values are those inter() forms).
 struct QuickCoef {
-    double xi, k, rk, r1k, rkm1;
+    double xi, k;
+};
+// The same with the reciprocals of k, 1 - k, k - 1.  On a grid whose spacings
+// are powers of two k = -1, so the divisions of inter() by k, 1 - k and k - 1
+// are by powers of two: multiplying by the exact reciprocal then rounds to the
+// same double as dividing, and the kernel of such grids takes that form.
+struct QuickExact : QuickCoef {
+    double rk, r1k, rkm1;
 };
 // Per axis, index t = ii + ng: Q[4t + 0] own axis, vel > 0; 4t + 1 own
 // axis, otherwise; 4t + 2 cross axis, vel > 0; 4t + 3 cross axis, otherwise.
@@ -48,18 +51,17 @@ struct MomTab {
 };
 
 // inter(x0,x1,x2,x,y0,y1,y2), paris.f90:2390-2411 (QUICK branch), with the
-// coordinate part from the table
-template <bool R>
+// coordinate part from the table, dividing or by the exact reciprocals
 __device__ inline double inter_q(const QuickCoef* __restrict__ c, double y0, double y1, double y2) {
     const double k = c->k, xi = c->xi;
-    double a, b;
-    if (R) {
-        a = ((y2 - k * k * y1 + (k * k - 1.0) * y0) * c->rk) * c->r1k;
-        b = ((y2 - k * y1 + (k - 1.0) * y0) * c->rk) * c->rkm1;
-    } else {
-        a = (y2 - k * k * y1 + (k * k - 1.0) * y0) / k / (1.0 - k);
-        b = (y2 - k * y1 + (k - 1.0) * y0) / k / (k - 1.0);
-    }
+    const double a = (y2 - k * k * y1 + (k * k - 1.0) * y0) / k / (1.0 - k);
+    const double b = (y2 - k * y1 + (k - 1.0) * y0) / k / (k - 1.0);
+    return y0 + a * xi + b * (xi * xi);
+}
+__device__ inline double inter_exact(const QuickExact& c, double y0, double y1, double y2) {
+    const double k = c.k, xi = c.xi;
+    const double a = ((y2 - k * k * y1 + (k * k - 1.0) * y0) * c.rk) * c.r1k;
+    const double b = ((y2 - k * y1 + (k - 1.0) * y0) * c.rk) * c.rkm1;
     return y0 + a * xi + b * (xi * xi);
 }
 
@@ -73,32 +75,35 @@ __device__ inline double quick_same(const double* __restrict__ phi, long n, long
     const double pm2 = phi[n - 2 * st], pm1 = phi[n - st], p0 = phi[n], pp1 = phi[n + st];
     const bool up = pm1 + p0 > 0.0;
     const double y2 = up ? pm2 : pp1;
-    return inter_q<false>(Q + 4 * t + (up ? 0 : 1), up ? pm1 : p0, up ? p0 : pm1, y2);
+    return inter_q(Q + 4 * t + (up ? 0 : 1), up ? pm1 : p0, up ? p0 : pm1, y2);
 }
 // the same with the two coefficient sets of a uniform axis
 __device__ inline QuickCoef pick(bool up, const QuickCoef& a, const QuickCoef& b) {
-    return QuickCoef{up ? a.xi : b.xi, up ? a.k : b.k, up ? a.rk : b.rk, up ? a.r1k : b.r1k, up ? a.rkm1 : b.rkm1};
+    return QuickCoef{up ? a.xi : b.xi, up ? a.k : b.k};
 }
-// inter_q<true> for the coefficients of every face of a uniform grid whose
+__device__ inline QuickExact pick(bool up, const QuickExact& a, const QuickExact& b) {
+    return QuickExact{{up ? a.xi : b.xi, up ? a.k : b.k}, up ? a.rk : b.rk, up ? a.r1k : b.r1k, up ? a.rkm1 : b.rkm1};
+}
+// inter_exact for the coefficients of every face of a uniform grid whose
 // coordinates are exact (xi = 1/2, k = -1, so k*k = 1, k*k - 1 = 0, k - 1 = -2,
 // 1/k = -1, 1/(1-k) = 1/2, 1/(k-1) = -1/2): the same IEEE operations with
 // those constants, the exact products by -1 folded into the scalings
-// ((x * -1) * 1/2 and x * -1/2 round alike), so the same double as inter_q
+// ((x * -1) * 1/2 and x * -1/2 round alike), so the same double as inter_exact
 __device__ inline double inter_canon(double y0, double y1, double y2) {
     const double a = ((y2 - y1) + 0.0 * y0) * -0.5;
     const double b = ((y2 + y1) + -2.0 * y0) * 0.5;
     return (y0 + a * 0.5) + b * 0.25;
 }
 template <bool C>
-__device__ inline double inter_u(const QuickCoef& c, double y0, double y1, double y2) {
-    return C ? inter_canon(y0, y1, y2) : inter_q<true>(&c, y0, y1, y2);
+__device__ inline double inter_u(const QuickExact& c, double y0, double y1, double y2) {
+    return C ? inter_canon(y0, y1, y2) : inter_exact(c, y0, y1, y2);
 }
 template <bool C>
-__device__ inline double quick_same_u(const double* __restrict__ phi, long n, long st, const QuickCoef& cu,
-                                      const QuickCoef& cd) {
+__device__ inline double quick_same_u(const double* __restrict__ phi, long n, long st, const QuickExact& cu,
+                                      const QuickExact& cd) {
     const double pm2 = phi[n - 2 * st], pm1 = phi[n - st], p0 = phi[n], pp1 = phi[n + st];
     const bool up = pm1 + p0 > 0.0;
-    const QuickCoef c = C ? cu : pick(up, cu, cd);
+    const QuickExact c = C ? cu : pick(up, cu, cd);
     return inter_u<C>(c, up ? pm1 : p0, up ? p0 : pm1, up ? pm2 : pp1);
 }
 
@@ -109,15 +114,15 @@ __device__ inline double quick_cross(const double* __restrict__ phi, const doubl
     const double v0 = vel[n], v1 = vel[n + sc];
     const double am = phi[n - st], a = phi[n], b = phi[n + st], bp = phi[n + 2 * st];
     const bool up = v0 + v1 > 0.0;
-    return inter_q<false>(Q + 4 * t + (up ? 2 : 3), up ? a : b, up ? b : a, up ? am : bp);
+    return inter_q(Q + 4 * t + (up ? 2 : 3), up ? a : b, up ? b : a, up ? am : bp);
 }
 template <bool C>
 __device__ inline double quick_cross_u(const double* __restrict__ phi, const double* __restrict__ vel, long n, long st,
-                                       long sc, const QuickCoef& cu, const QuickCoef& cd) {
+                                       long sc, const QuickExact& cu, const QuickExact& cd) {
     const double v0 = vel[n], v1 = vel[n + sc];
     const double am = phi[n - st], a = phi[n], b = phi[n + st], bp = phi[n + 2 * st];
     const bool up = v0 + v1 > 0.0;
-    const QuickCoef c = C ? cu : pick(up, cu, cd);
+    const QuickExact c = C ? cu : pick(up, cu, cd);
     return inter_u<C>(c, up ? a : b, up ? b : a, up ? am : bp);
 }
 
@@ -125,7 +130,7 @@ __device__ inline double quick_cross_u(const double* __restrict__ phi, const dou
 // coefficient sets and metric reciprocals per axis (checked bit for bit on
 // the host), passed by value so the kernel loads no table.
 struct QuickUniform {
-    QuickCoef q[3][4];
+    QuickExact q[3][4];
     double d[3], dh[3], rd[3], rdh[3];
 };
 
@@ -139,7 +144,7 @@ struct QuickUniform {
 // twelve face values per cell instead of eighteen.  An outer lane forms only
 // what its neighbour takes, at cells within the ghost layers' stencil reach.
 // The coefficients of the x axis, different in every lane, stay in registers
-// (as table rows of 160 bytes they took a sector per lane in every face value).
+// (as table rows they took a sector per lane in every face value).
 // Warps in flight count for more than registers: eight blocks of 128 per SM (64
 // registers, some spilled) 425 us at 200x168x121, 479 with six, 529 with four,
 // 604 with a thread per cell and eighteen face values.
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(128, 8) k_conv_quick(Vel V, double* __restrict
         const double pm2 = phi[n - 2 * st], pm1 = phi[n - st], p0 = phi[n], pp1 = phi[n + st];
         const bool up = pm1 + p0 > 0.0;
         const QuickCoef c = pick(up, qx[0], qx[1]);
-        return inter_q<false>(&c, up ? pm1 : p0, up ? p0 : pm1, up ? pm2 : pp1);
+        return inter_q(&c, up ? pm1 : p0, up ? p0 : pm1, up ? pm2 : pp1);
     };
     // the value of phi on the face + 1/2 of axis a, upwinded by vel(n) + vel(n + sc)
     auto cross = [&](const double* phi, const double* vel, long n, int a, long sc, int t) {
@@ -181,7 +186,7 @@ __global__ void __launch_bounds__(128, 8) k_conv_quick(Vel V, double* __restrict
         const double am = phi[n - st], p = phi[n], b = phi[n + st], bp = phi[n + 2 * st];
         const bool up = v0 + v1 > 0.0;
         const QuickCoef c = pick(up, qx[2], qx[3]);
-        return inter_q<false>(&c, up ? p : b, up ? b : p, up ? am : bp);
+        return inter_q(&c, up ? p : b, up ? b : p, up ? am : bp);
     };
     auto by_d = [&](double x, int a, int t) { return x / (a == 0 ? ddx : G.a[a].d[t]); };
     auto by_dh = [&](double x, int a, int t) { return x / (a == 0 ? ddxh : G.a[a].dh[t]); };
@@ -488,7 +493,7 @@ bool pow2(double x) {
 
 // The per-index tables of MomTab, built once per grid on the host from the
 // host copies of the coordinates (the same doubles the device holds).
-int mom_tables(paris_ctx* c, MomTab* T, bool* exact, QuickUniform* U = nullptr, bool* uniform = nullptr) {
+int mom_tables(paris_ctx* c, MomTab* T, QuickUniform* U, bool* uniform) {
     const int g = c->L.ng;
     const std::vector<double>* C[3] = {&c->h_x, &c->h_y, &c->h_z};
     const std::vector<double>* H[3] = {&c->h_xh, &c->h_yh, &c->h_zh};
@@ -513,11 +518,7 @@ int mom_tables(paris_ctx* c, MomTab* T, bool* exact, QuickUniform* U = nullptr, 
             auto set = [&](QuickCoef& q, double x0, double x1, double x2, double xx, bool used) {
                 q.xi = (xx - x0) / (x1 - x0);
                 q.k = (x2 - x0) / (x1 - x0);
-                const double omk = 1.0 - q.k, km1 = q.k - 1.0;
-                q.rk = 1.0 / q.k;
-                q.r1k = 1.0 / omk;
-                q.rkm1 = 1.0 / km1;
-                if (used) ex = ex && pow2(q.k) && pow2(omk) && pow2(km1);
+                if (used) ex = ex && pow2(q.k) && pow2(1.0 - q.k) && pow2(q.k - 1.0);
             };
             for (int t = 0; t < nt; t++) {
                 // own axis: ii = t - g in [0, n]; cross axis: jj = t - g in [-1, n-1]
@@ -541,45 +542,42 @@ int mom_tables(paris_ctx* c, MomTab* T, bool* exact, QuickUniform* U = nullptr, 
         T->rd[a] = c->mom_tab + off[a] + 4L * per * nt;
         T->rdh[a] = T->rd[a] + nt;
     }
-    *exact = c->mom_tab_exact != 0;
-    if (uniform) {
-        // every index the kernel reads holds the same coefficients, bit for bit
-        // (then rebuilt here from the host coordinates: same arithmetic)
-        bool uni = *exact;
-        for (int a = 0; a < 3 && uni; a++) {
-            const std::vector<double>&x = *C[a], &xh = *H[a], &d = *D[a], &dh = *DH[a];
-            const int n = c->L.n[a];
-            auto coef = [&](int v, int t) {
-                QuickCoef q;
-                double x0, x1, x2, xx;
-                if (v == 0) { x0 = xh[t - 1]; x1 = xh[t]; x2 = xh[t - 2]; xx = x[t]; }
-                else if (v == 1) { x0 = xh[t]; x1 = xh[t - 1]; x2 = xh[t + 1]; xx = x[t]; }
-                else if (v == 2) { x0 = x[t]; x1 = x[t + 1]; x2 = x[t - 1]; xx = xh[t]; }
-                else { x0 = x[t + 1]; x1 = x[t]; x2 = x[t + 2]; xx = xh[t]; }
-                q.xi = (xx - x0) / (x1 - x0);
-                q.k = (x2 - x0) / (x1 - x0);
-                q.rk = 1.0 / q.k;
-                q.r1k = 1.0 / (1.0 - q.k);
-                q.rkm1 = 1.0 / (q.k - 1.0);
-                return q;
-            };
-            auto same = [](const QuickCoef& p, const QuickCoef& q) {
-                return p.xi == q.xi && p.k == q.k && p.rk == q.rk && p.r1k == q.r1k && p.rkm1 == q.rkm1;
-            };
-            for (int v = 0; v < 4; v++) {
-                const int t0 = v < 2 ? g : g - 1, t1 = v < 2 ? n + g : n + g - 1;
-                U->q[a][v] = coef(v, t0);
-                for (int t = t0 + 1; t <= t1 && uni; t++) uni = same(coef(v, t), U->q[a][v]);
-            }
-            U->d[a] = d[g];
-            U->dh[a] = dh[g];
-            // explicitMomDiff reads the metric one index beyond the interior
-            for (int t = g - 1; t <= n + g && uni; t++) uni = d[t] == d[g] && dh[t] == dh[g];
-            U->rd[a] = 1. / d[g];
-            U->rdh[a] = 1. / dh[g];
+    // exact, and every index the kernel reads holds the same coefficients, bit
+    // for bit (rebuilt here from the host coordinates: same arithmetic)
+    bool uni = c->mom_tab_exact != 0;
+    for (int a = 0; a < 3 && uni; a++) {
+        const std::vector<double>&x = *C[a], &xh = *H[a], &d = *D[a], &dh = *DH[a];
+        const int n = c->L.n[a];
+        auto coef = [&](int v, int t) {
+            QuickExact q;
+            double x0, x1, x2, xx;
+            if (v == 0) { x0 = xh[t - 1]; x1 = xh[t]; x2 = xh[t - 2]; xx = x[t]; }
+            else if (v == 1) { x0 = xh[t]; x1 = xh[t - 1]; x2 = xh[t + 1]; xx = x[t]; }
+            else if (v == 2) { x0 = x[t]; x1 = x[t + 1]; x2 = x[t - 1]; xx = xh[t]; }
+            else { x0 = x[t + 1]; x1 = x[t]; x2 = x[t + 2]; xx = xh[t]; }
+            q.xi = (xx - x0) / (x1 - x0);
+            q.k = (x2 - x0) / (x1 - x0);
+            q.rk = 1.0 / q.k;
+            q.r1k = 1.0 / (1.0 - q.k);
+            q.rkm1 = 1.0 / (q.k - 1.0);
+            return q;
+        };
+        auto same = [](const QuickExact& p, const QuickExact& q) {
+            return p.xi == q.xi && p.k == q.k && p.rk == q.rk && p.r1k == q.r1k && p.rkm1 == q.rkm1;
+        };
+        for (int v = 0; v < 4; v++) {
+            const int t0 = v < 2 ? g : g - 1, t1 = v < 2 ? n + g : n + g - 1;
+            U->q[a][v] = coef(v, t0);
+            for (int t = t0 + 1; t <= t1 && uni; t++) uni = same(coef(v, t), U->q[a][v]);
         }
-        *uniform = uni;
+        U->d[a] = d[g];
+        U->dh[a] = dh[g];
+        // explicitMomDiff reads the metric one index beyond the interior
+        for (int t = g - 1; t <= n + g && uni; t++) uni = d[t] == d[g] && dh[t] == dh[g];
+        U->rd[a] = 1. / d[g];
+        U->rdh[a] = 1. / dh[g];
     }
+    *uniform = uni;
     return PARIS_OK;
 }
 
@@ -601,8 +599,8 @@ extern "C" int paris_momentum_convection(paris_handle_t c, int32_t scheme) {
     if (scheme == PARIS_CONV_QUICK) {
         MomTab T;
         QuickUniform U;
-        bool exact, uniform;
-        PARIS_CHECK(mom_tables(c, &T, &exact, &U, &uniform));
+        bool uniform;
+        PARIS_CHECK(mom_tables(c, &T, &U, &uniform));
         bool canon = uniform;   // every coefficient set xi = 1/2, k = -1 exactly
         for (int a = 0; a < 3 && canon; a++)
             for (int v = 0; v < 4; v++) canon = canon && U.q[a][v].xi == 0.5 && U.q[a][v].k == -1.0;
@@ -635,8 +633,8 @@ extern "C" int paris_explicit_mom_diff(paris_handle_t c) {
     PARIS_CHECK(need(c, {PARIS_FIELD_MU, PARIS_FIELD_DU, PARIS_FIELD_DV, PARIS_FIELD_DW}));
     MomTab T;
     QuickUniform U;
-    bool exact, uniform;
-    PARIS_CHECK(mom_tables(c, &T, &exact, &U, &uniform));
+    bool uniform;
+    PARIS_CHECK(mom_tables(c, &T, &U, &uniform));
     if (uniform)
         PARIS_LAUNCH_N(c, "mom_diffusion", c->N, k_mom_diff<true>, cgrid(c->L), cblock(), 0, vel(c),
                        c->fld[PARIS_FIELD_RHO], c->fld[PARIS_FIELD_MU], c->fld[PARIS_FIELD_DU], c->fld[PARIS_FIELD_DV],
