@@ -45,6 +45,29 @@ def test_convection_bitwise(gpu_lib, capi, runtime, orc, bc, scheme, grid):
         assert (b != s).any()
 
 
+# QUICK with divisions takes x tiles of 30 cells whose faces pass between lanes,
+# and marches along z in chunks of 4, 8 or 16 planes: one tile filled, a last
+# tile of one cell and of five, odd rows; chunks of 8 and 16 with a partial last one
+@pytest.mark.parametrize("bc", ["periodic", "wall", "mixed"])
+@pytest.mark.parametrize("n", [(30, 7, 9), (31, 13, 10), (61, 9, 6), (95, 5, 11), (61, 93, 133), (95, 131, 150)])
+def test_quick_tiles_and_chunks_bitwise(gpu_lib, capi, runtime, orc, n, bc):
+    P, W = capi.BC_PERIODIC, capi.BC_WALL
+    d = capi.make_desc(n, bc=[W, P, W, W, P, W] if bc == "mixed" else bc)
+    rng = np.random.default_rng(6)
+    u, v, w = (rng.standard_normal(orc.shape(d)) for _ in range(3))
+    orc.set_velocity_bc(d, u, v, w)
+    sentinel = [orc.zeros(d) + 7.0 + q for q in range(3)]   # entries the scheme leaves alone stay
+    ref = [a.copy() for a in sentinel]
+    assert orc.momentum_convection(d, 0, u, v, w, *ref) == 0
+    with runtime.ParisGpu(d) as gpu:
+        upload(gpu, capi, u=u, v=v, w=w, du=sentinel[0], dv=sentinel[1], dw=sentinel[2])
+        gpu.momentum_convection(0)
+        out = [gpu.download(f) for f in (capi.F_DU, capi.F_DV, capi.F_DW)]
+    for a, b, s in zip(out, ref, sentinel):
+        assert np.array_equal(a, b)
+        assert (b != s).any()
+
+
 @pytest.mark.parametrize("grid", ["general", "pow2"])
 @pytest.mark.parametrize("bc", ["periodic", "wall"])
 def test_diffusion_force_advance_bitwise(gpu_lib, capi, runtime, orc, bc, grid):
