@@ -9,10 +9,11 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def state(capi, orc, bc, seed):
-    n = 24
-    d = capi.make_desc((n, n + 4, n - 4), bc=bc, rho1=1.2, rho2=1000.0, mu1=1.8e-5, mu2=1e-3,
-                       length=(1.0, 28 / 24, 20 / 24))
+def state(capi, orc, bc, seed, grid="general"):
+    # "pow2": spacings 1/16, 1/32 and 1/4, all different, where the vorticity is
+    # formed with their exact reciprocals; "general": cells of 1/24, where it divides
+    n, length = ((16, 32, 8), (1.0, 1.0, 2.0)) if grid == "pow2" else ((24, 28, 20), (1.0, 28 / 24, 20 / 24))
+    d = capi.make_desc(n, bc=bc, rho1=1.2, rho2=1000.0, mu1=1.8e-5, mu2=1e-3, length=length)
     rng = np.random.default_rng(seed)
     cvof, flag, _ = orc.init_spheres(d, [(0.45, 0.6, 0.4), (0.7, 0.3, 0.45)], [0.2, 0.12], refinement=4)
     f = {"cvof": cvof, "flag": flag}
@@ -41,10 +42,11 @@ def scale(d, ab):
     return s
 
 
+@pytest.mark.parametrize("grid", ["general", "pow2"])
 @pytest.mark.parametrize("bc", ["wall", "periodic"])
 @pytest.mark.parametrize("flags", [0, 1, 6])
-def test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags):
-    d, f = state(capi, orc, bc, 5)
+def test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags, grid):
+    d, f = state(capi, orc, bc, 5, grid)
     o = capi.make_stats_opts(dpdx=(0.2, -0.1, 0.05), gravity=(0.0, -9.81, 0.3), buoyancy=3, rho_ave=400.0,
                              test_flags=flags)
     ref, ab = orc.calc_stats(d, f["u"], f["v"], f["w"], f["rho"], f["p"], f["cvof"], f["mu"], f["flag"], o)
