@@ -22,7 +22,7 @@
 // sweep of the post-smoothing pair).
 #pragma once
 
-// the configurations the solver uses
+// the configurations of the opt-in form
 template <typename T>
 struct SwGeo4;
 template <>

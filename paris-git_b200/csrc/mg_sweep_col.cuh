@@ -37,9 +37,10 @@
 // What bounds it: on the finest level, instruction issue and HBM together.
 // Scalar shared-memory operands and two barriers per pair of planes held the
 // earlier form to 138 us per FP32 256^3 sweep (2.9 TB/s of its 24 B/cell); this
-// one takes 87 us (4.6 TB/s), 65 from a zero iterate, at
-// 268 instructions per warp and step of 128 cells (436 with run-time row pitches,
-// register copies and a branch on the parity in every step).  On the lower
+// one takes 84 us (4.8 TB/s), 65 from a zero iterate, 104 with the correction, at
+// 263 instructions per warp and step of 128 cells (436 with run-time row pitches,
+// register copies and a branch on the parity in every step; 87 and 110 us with
+// the new F values stored into the staged planes).  On the lower
 // levels, resident in L2, the depth of the march: (planes per block + 2) steps.
 // Requirements (checked by the host): n0 a multiple of 4, n1 and n2 even, fewer
 // than 2^32 cells.

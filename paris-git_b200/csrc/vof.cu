@@ -205,7 +205,7 @@ __device__ inline double cell_flux(const SweepArgs& a, double cc, long n, double
 // :731-745 and get_flags_and_clip) and the flag, into the second buffer.
 // Each thread updates kVofUpd cells of a row, a block's width apart; the width
 // covers the row with few idle lanes (150 cells: one block of 96 threads, 215 to
-// 198 us for three sweeps of 150x93x121).  The volume fractions and face
+// 198 us for two steps of three sweeps of 150x93x121).  The volume fractions and face
 // velocities of all its cells are loaded before any test on them, so their loads
 // are in flight together.
 static constexpr int kVofUpdThreads = 128, kVofUpd = 2;

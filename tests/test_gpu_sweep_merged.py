@@ -1,10 +1,10 @@
 """The fused sweep with merged phases (one barrier per step) against the
-default two-phase form.
+solver's own column sweep.
 
 Both run the same updates in the same order for every cell; the merged form
 runs the second colour of one step and the first colour of the next between
-the same two barriers, on 32x12 (PARIS_SWEEP_MERGED=1) or 32x14 (2) tiles,
-against 32x16.  A defect-correction solve therefore gives the same pressure
+the same two barriers, on 32x12 (PARIS_SWEEP_MERGED=1) or 32x14 (2) tiles.  A
+defect-correction solve therefore gives the same pressure
 to the bit, a CG solve the same to rounding (its r.z partials come from other
 tiles: assert_same_solve).  The environment variable is read when a handle
 first builds its FP32 multigrid levels.  Grids: periodic and walled boxes

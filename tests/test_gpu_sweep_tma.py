@@ -1,11 +1,10 @@
-"""The TMA-staged fused sweep against the cp.async-staged one.
+"""The TMA-staged fused sweep against the solver's own column sweep.
 
-The two kernels share the tiles, the wavefront and the arithmetic of the
-fused red-black sweep and differ only in how the planes reach shared memory,
-so a defect-correction solve with either gives the same pressure to the bit
+The two kernels do the same updates with the same arithmetic, so a
+defect-correction solve with either gives the same pressure to the bit
 (a CG solve the same to rounding: assert_same_solve).  The
 environment variable PARIS_SWEEP_TMA, read when a handle first builds its
-FP32 multigrid levels, selects the TMA staging (1) or the cp.async one (0,
+FP32 multigrid levels, selects the TMA form (1) or the column sweep (0,
 the default); both arms run the sweeps one at a time (PARIS_SWEEP_PAIRS=0).
 Grids: periodic and walled boxes, and mixed boundaries, whose fused levels
 (at least 32^3 cells) have the first and last tiles of every row and column
