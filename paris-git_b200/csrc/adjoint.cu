@@ -132,7 +132,7 @@ extern "C" int paris_projection_adjoint(paris_handle_t c, double dt, const doubl
     }
     cudaSetDevice(c->dev);
     const long T = c->L.total;
-    if (!c->adj) PARIS_CUDA_TRY(c, cudaMalloc(&c->adj, (10 * T + c->N) * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, &c->adj, (10 * T + c->N) * sizeof(double)));
     double* w[3] = {c->adj, c->adj + T, c->adj + 2 * T};
     double* lam = c->adj + 3 * T;
     double* so[3] = {c->adj + 4 * T, c->adj + 5 * T, c->adj + 6 * T};

@@ -167,6 +167,7 @@ void ctx_set_error(paris_ctx* c, const char* fmt, ...);
     do {                                                                            \
         cudaError_t _e = (expr);                                                    \
         if (_e != cudaSuccess) {                                                    \
+            cudaGetLastError();   /* or the next launch would report it */          \
             ctx_set_error((ctx), "%s failed: %s (%s:%d)", #expr,                    \
                           cudaGetErrorString(_e), __FILE__, __LINE__);              \
             return PARIS_CUDA_ERROR;                                                \

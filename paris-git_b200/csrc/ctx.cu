@@ -32,8 +32,21 @@ static void make_axis(int n, int ng, double L, std::vector<double>& x, std::vect
     dx[0] = dx[1];
 }
 
+int ctx_malloc_bytes(paris_ctx* c, void** p, size_t bytes) {
+    if (*p) return PARIS_OK;
+    void* q = nullptr;
+    const cudaError_t e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // or the next launch would report it
+        ctx_set_error(c, "no device memory for %zu bytes: %s", bytes, cudaGetErrorString(e));
+        return PARIS_CUDA_ERROR;
+    }
+    *p = q;
+    return PARIS_OK;
+}
+
 static int upload_vec(paris_ctx* c, double** d, const std::vector<double>& h) {
-    PARIS_CUDA_TRY(c, cudaMalloc(d, h.size() * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, d, h.size() * sizeof(double)));
     PARIS_CUDA_TRY(c, cudaMemcpy(*d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
     return PARIS_OK;
 }
@@ -41,14 +54,14 @@ static int upload_vec(paris_ctx* c, double** d, const std::vector<double>& h) {
 int ctx_alloc_field(paris_ctx* c, int field) {
     if (field == PARIS_FIELD_VOF_FLAG) {
         if (!c->flag) {
-            PARIS_CUDA_TRY(c, cudaMalloc(&c->flag, c->L.total));
+            PARIS_CHECK(ctx_malloc(c, &c->flag, c->L.total));
             PARIS_CUDA_TRY(c, cudaMemsetAsync(c->flag, 0, c->L.total, c->stream));
         }
         return PARIS_OK;
     }
     if (field == PARIS_FIELD_HEIGHT) {
         if (!c->height) {
-            PARIS_CUDA_TRY(c, cudaMalloc(&c->height, 6 * c->L.total * sizeof(double)));
+            PARIS_CHECK(ctx_malloc(c, &c->height, 6 * c->L.total * sizeof(double)));
             PARIS_CUDA_TRY(c, cudaMemsetAsync(c->height, 0, 6 * c->L.total * sizeof(double), c->stream));
         }
         return PARIS_OK;
@@ -56,7 +69,7 @@ int ctx_alloc_field(paris_ctx* c, int field) {
     if (field == PARIS_FIELD_A || field == PARIS_FIELD_VOF_PHASE) return PARIS_OK;
     if (field < 0 || field >= PARIS_NFIELDS) return PARIS_BAD_ARGS;
     if (!c->fld[field]) {
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->fld[field], c->L.total * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->fld[field], c->L.total * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMemsetAsync(c->fld[field], 0, c->L.total * sizeof(double), c->stream));
     }
     return PARIS_OK;
@@ -252,6 +265,7 @@ extern "C" int paris_gpu_init(const paris_grid_desc* desc, paris_handle_t* out) 
     if (!s && cudaStreamSynchronize(c->stream) != cudaSuccess) s = PARIS_CUDA_ERROR;
     if (s) {
         paris_gpu_finalize(c);
+        cudaGetLastError();   // or another handle's next launch would report it
         return s;
     }
     *out = c;
@@ -302,7 +316,7 @@ extern "C" int paris_gpu_finalize(paris_handle_t c) {
 static int ensure_stage(paris_ctx* c) {
     if (!c->i32stage) {
         long nt = (long)(c->d.nx + 4) * (c->d.ny + 4) * (c->d.nz + 4);
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->i32stage, nt * sizeof(int32_t)));
+        PARIS_CHECK(ctx_malloc(c, &c->i32stage, nt * sizeof(int32_t)));
     }
     return PARIS_OK;
 }
@@ -333,7 +347,7 @@ extern "C" int paris_gpu_upload(paris_handle_t c, int32_t field, const void* hos
     } else if (field == PARIS_FIELD_VOF_PHASE) {
         return PARIS_BAD_ARGS;   // derived from cvof
     } else if (field == PARIS_FIELD_A) {
-        if (!c->A) PARIS_CUDA_TRY(c, cudaMalloc(&c->A, 8 * c->N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->A, 8 * c->N * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMemcpyAsync(c->A, host, 8 * c->N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
         c->A_valid = 1;
         c->A_from_upload = 1;
@@ -417,7 +431,7 @@ static int async_setup(paris_ctx* c, int f, bool in) {
     }
     double** buf = in ? &c->stage_in[f] : &c->stage_out[f];
     if (!*buf) {
-        PARIS_CUDA_TRY(c, cudaMalloc(buf, c->L.total * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, buf, c->L.total * sizeof(double)));
         cudaEvent_t* e0 = in ? &c->ev_in_done[f] : &c->ev_out_ready[f];
         cudaEvent_t* e1 = in ? &c->ev_in_free[f] : &c->ev_out_free[f];
         PARIS_CUDA_TRY(c, cudaEventCreateWithFlags(e0, cudaEventDisableTiming));
@@ -570,11 +584,6 @@ extern "C" int64_t paris_gpu_profile_report(paris_handle_t c, char* buf, int64_t
 }
 
 int ctx_ensure_matrix(paris_ctx* c) {
-    if (!c->cx) {
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->cx, c->N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->cy, c->N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->cz, c->N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->rhs, c->N * sizeof(double)));
-    }
+    for (double** p : {&c->cx, &c->cy, &c->cz, &c->rhs}) PARIS_CHECK(ctx_malloc(c, p, c->N * sizeof(double)));
     return PARIS_OK;
 }

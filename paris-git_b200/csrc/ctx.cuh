@@ -12,10 +12,10 @@ static constexpr int kRedBlocks = 1184;   // 148 SMs x 8: capacity of the partia
 struct RefLevel {
     int n[3];
     long N;
-    double* K;   // 8*N
-    double* p;   // pMG
-    double* e;   // EMG
-    double* q;   // beta / K7
+    double* K = nullptr;   // 8*N
+    double* p = nullptr;   // pMG
+    double* e = nullptr;   // EMG
+    double* q = nullptr;   // beta / K7
 };
 
 // Geometry of a launch of the column sweep: W output cells across a tile, H ring
@@ -32,9 +32,9 @@ template <typename T>
 struct FastLevel {
     int n[3];
     long N;
-    T *cx, *cy, *cz;
-    T *b, *x;
-    T* x2;   // second iterate of the fused sweeps (they read one and write the other)
+    T *cx = nullptr, *cy = nullptr, *cz = nullptr;
+    T *b = nullptr, *x = nullptr;
+    T* x2 = nullptr;   // second iterate of the fused sweeps (they read one and write the other)
     void* tma = nullptr;   // FP32: tensor maps of the level for the TMA-staged sweep (mg_fast.cu)
     bool pairs = false;    // two consecutive sweeps run as one pass (k_rb_sweep4_cfg)
     bool rs = false;       // the last pre-smoothing sweep forms the coarse right-hand side (k_rb_sweep_rs)
@@ -137,6 +137,14 @@ struct paris_ctx {
     std::vector<cudaEvent_t> evpool;
 };
 
+
+// Device memory at *p, if it is not there yet.  After a failure *p is null, so
+// that the next call that needs it tries again.
+int ctx_malloc_bytes(paris_ctx* c, void** p, size_t bytes);
+template <typename T>
+int ctx_malloc(paris_ctx* c, T** p, size_t bytes) {
+    return ctx_malloc_bytes(c, (void**)p, bytes);
+}
 
 // Resident blocks per SM of a kernel with smem bytes of dynamic shared memory
 // (0: the device refuses it; the error is set).  Lifts the kernel's limit of

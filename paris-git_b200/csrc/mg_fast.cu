@@ -899,9 +899,8 @@ static int sweep_col_choose(const paris_ctx* c, FastLevel<T>& l) {
 }
 
 template <typename T>
-static int fast_alloc(paris_ctx* c) {
+static int fast_levels(paris_ctx* c) {
     auto& lv = levels<T>(c);
-    if (!lv.empty()) return PARIS_OK;
     int nl = fast_depth(c);
     c->fast_nl = nl;
     lv.resize(nl);
@@ -909,13 +908,12 @@ static int fast_alloc(paris_ctx* c) {
         FastLevel<T>& l = lv[L];
         l.n[0] = c->d.nx >> L; l.n[1] = c->d.ny >> L; l.n[2] = c->d.nz >> L;
         l.N = (long)l.n[0] * l.n[1] * l.n[2];
-        for (T** p : {&l.cx, &l.cy, &l.cz, &l.b, &l.x}) PARIS_CUDA_TRY(c, cudaMalloc(p, l.N * sizeof(T)));
+        for (T** p : {&l.cx, &l.cy, &l.cz, &l.b, &l.x}) PARIS_CHECK(ctx_malloc(c, p, l.N * sizeof(T)));
         // the fused sweep stages 16-byte row chunks and pairs cells by parity
-        l.x2 = nullptr;
         bool fusable = l.N >= kFusedCells && l.N > kCoarseCells && l.n[0] % 4 == 0 && l.n[1] % 2 == 0 &&
                        l.n[2] % 2 == 0 && L < nl - 1 && l.N < 1L << 32;
         if (fusable) {
-            PARIS_CUDA_TRY(c, cudaMalloc(&l.x2, l.N * sizeof(T)));
+            PARIS_CHECK(ctx_malloc(c, &l.x2, l.N * sizeof(T)));
             PARIS_CHECK(sweep_col_choose(c, l));
         }
         l.pairs = fusable && pairs_wanted();
@@ -924,6 +922,23 @@ static int fast_alloc(paris_ctx* c) {
         if constexpr (std::is_same<T, float>::value) level_maps(l);
     }
     return PARIS_OK;
+}
+
+// all levels or, where memory does not last, none
+template <typename T>
+static int fast_alloc(paris_ctx* c) {
+    auto& lv = levels<T>(c);
+    if (!lv.empty()) return PARIS_OK;
+    const int st = fast_levels<T>(c);
+    if (st != PARIS_OK) {
+        if (std::is_same<T, float>::value) mg_fast_free_maps(c);
+        for (FastLevel<T>& l : lv) {
+            T* const all[] = {l.cx, l.cy, l.cz, l.b, l.x, l.x2};
+            for (T* p : all) cudaFree(p);
+        }
+        lv.clear();
+    }
+    return st;
 }
 
 template <typename T>
@@ -1250,7 +1265,7 @@ static int solve_dc(paris_ctx* c, const paris_solve_opts* o, paris_solve_result*
 // read uninitialised memory (0 * NaN is NaN)
 static int alloc_vec(paris_ctx* c, double** p) {
     if (!*p) {
-        PARIS_CUDA_TRY(c, cudaMalloc(p, c->N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, p, c->N * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMemsetAsync(*p, 0, c->N * sizeof(double), c->stream));
     }
     return PARIS_OK;

@@ -298,8 +298,7 @@ __global__ void k_ref_field_io(double* __restrict__ pf, double* __restrict__ pm,
 
 static LvlDims dims(const RefLevel& l) { return LvlDims{l.n[0], l.n[1], l.n[2], l.N}; }
 
-static int ref_alloc(paris_ctx* c) {
-    if (!c->ref.empty()) return PARIS_OK;
+static int ref_levels(paris_ctx* c) {
     int nd[3] = {c->d.nx, c->d.ny, c->d.nz};
     int lmg = 1000;
     for (int a = 0; a < 3; a++) {
@@ -311,19 +310,35 @@ static int ref_alloc(paris_ctx* c) {
         while ((1 << (L + 1)) <= nd[a]) L++;
         lmg = L < lmg ? L : lmg;
     }
-    if (lmg < 2 || lmg > kRefMaxLevels || c->N > 1L << 30) return PARIS_BAD_ARGS;
+    if (lmg < 2 || lmg > kRefMaxLevels || c->N > 1L << 30) {
+        ctx_set_error(c, "multigrid of %d levels over %ld cells: 2 to %d levels and at most 2^30 cells", lmg, c->N,
+                      kRefMaxLevels);
+        return PARIS_BAD_ARGS;
+    }
     c->ref_lmg = lmg;
     c->ref.resize(lmg + 1);
     for (int L = lmg; L >= 1; L--) {
         RefLevel& l = c->ref[L];
         for (int a = 0; a < 3; a++) l.n[a] = nd[a] >> (lmg - L);
         l.N = (long)l.n[0] * l.n[1] * l.n[2];
-        PARIS_CUDA_TRY(c, cudaMalloc(&l.K, 8 * l.N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&l.p, l.N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&l.e, l.N * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&l.q, l.N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &l.K, 8 * l.N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &l.p, l.N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &l.e, l.N * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &l.q, l.N * sizeof(double)));
     }
     return PARIS_OK;
+}
+
+// all levels or, where memory does not last, none
+static int ref_alloc(paris_ctx* c) {
+    if (!c->ref.empty()) return PARIS_OK;
+    const int st = ref_levels(c);
+    if (st != PARIS_OK) {
+        for (RefLevel& l : c->ref)
+            for (double* p : {l.K, l.p, l.e, l.q}) cudaFree(p);
+        c->ref.clear();
+    }
+    return st;
 }
 
 static int log2_of(int n) {
@@ -338,7 +353,7 @@ static RefLvl ref_level(const RefLevel& l) {
 
 // one cycle: a cooperative launch, so that all its blocks are resident
 static int mg_iteration(paris_ctx* c, const RefCycle& C) {
-    if (!c->ref_bar) PARIS_CUDA_TRY(c, cudaMalloc(&c->ref_bar, 2 * sizeof(unsigned)));
+    PARIS_CHECK(ctx_malloc(c, &c->ref_bar, 2 * sizeof(unsigned)));
     PARIS_CUDA_TRY(c, cudaMemsetAsync(c->ref_bar, 0, 2 * sizeof(unsigned), c->stream));
     RefCycle a = C;
     void* args[] = {&a, &c->bnd, &c->ref_bar, &c->err_dev};

@@ -565,15 +565,15 @@ static int mc_wall_bc(paris_ctx* c, double* mom, const double* u, const double* 
 
 static int mc_alloc(paris_ctx* c) {
     const long nt = c->L.total;
-    if (!c->mc_tmp) {
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_tmp, nt * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_tmp2, nt * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_work, 3 * nt * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_fv, nt * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_flag, nt));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mc_cg, nt));
+    if (!c->mc_cg) {   // (the last of them)
+        PARIS_CHECK(ctx_malloc(c, &c->mc_tmp, nt * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->mc_tmp2, nt * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->mc_work, 3 * nt * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->mc_fv, nt * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->mc_flag, nt));
         PARIS_CUDA_TRY(c, cudaMemsetAsync(c->mc_fv, 0, nt * sizeof(double), c->stream));
         PARIS_CUDA_TRY(c, cudaMemsetAsync(c->mc_tmp2, 0, nt * sizeof(double), c->stream));
+        PARIS_CHECK(ctx_malloc(c, &c->mc_cg, nt));
     }
     return PARIS_OK;
 }

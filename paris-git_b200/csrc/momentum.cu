@@ -532,7 +532,7 @@ int mom_tables(paris_ctx* c, MomTab* T, QuickUniform* U, bool* uniform) {
                 if (t >= g && t < n + g) ex = ex && pow2(d[t]) && pow2(dh[t]);
             }
         }
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->mom_tab, total * sizeof(double)));
+        PARIS_CHECK(ctx_malloc(c, &c->mom_tab, total * sizeof(double)));
         PARIS_CUDA_TRY(c, cudaMemcpy(c->mom_tab, tab.data(), total * sizeof(double), cudaMemcpyHostToDevice));
         c->mom_tab_exact = ex ? 1 : 0;
     }

@@ -147,7 +147,7 @@ static bool uniform_pow2(const std::vector<double>& d, int n, int g, double* r) 
 
 int poisson_build_full_A(paris_ctx* c) {
     if (c->A_from_upload) { c->A_valid = 1; return PARIS_OK; }
-    if (!c->A) PARIS_CUDA_TRY(c, cudaMalloc(&c->A, 8 * c->N * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, &c->A, 8 * c->N * sizeof(double)));
     int with_mask = c->setup_dt != 0.0 ? 1 : 0;
     PARIS_LAUNCH(c, k_full_A, cell_grid(c->L), cell_block(), 0, c->fld[PARIS_FIELD_RHO], c->rhs, c->A, c->L,
                  c->bnd, metric(c), c->setup_dt, with_mask);

@@ -485,11 +485,9 @@ __global__ void __launch_bounds__(128) k_curv_pass2(const CurvArgs A) {
 static int curvatures(paris_ctx* c) {
     const Layout& L = c->L;
     PARIS_CHECK(ctx_alloc_field(c, PARIS_FIELD_KAPPA));
-    if (!c->kflag) PARIS_CUDA_TRY(c, cudaMalloc(&c->kflag, L.total));
-    if (!c->st_list) {
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->st_list, c->N * sizeof(int)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->st_count, sizeof(int)));
-    }
+    PARIS_CHECK(ctx_malloc(c, &c->kflag, L.total));
+    PARIS_CHECK(ctx_malloc(c, &c->st_list, c->N * sizeof(int)));
+    PARIS_CHECK(ctx_malloc(c, &c->st_count, sizeof(int)));
     CurvArgs A;
     A.s = st_args(c);
     A.kap = c->fld[PARIS_FIELD_KAPPA];

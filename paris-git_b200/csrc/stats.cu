@@ -230,10 +230,8 @@ extern "C" int paris_calc_stats(paris_handle_t c, const paris_stats_opts* opts, 
     for (int f : {PARIS_FIELD_U, PARIS_FIELD_V, PARIS_FIELD_W, PARIS_FIELD_RHO, PARIS_FIELD_P, PARIS_FIELD_CVOF,
                   PARIS_FIELD_MU, PARIS_FIELD_VOF_FLAG})
         PARIS_CHECK(ctx_alloc_field(c, f));
-    if (!c->stats_part) {
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->stats_part, (long)kNS * kRedBlocks * sizeof(double)));
-        PARIS_CUDA_TRY(c, cudaMalloc(&c->stats_out, kNS * sizeof(double)));
-    }
+    PARIS_CHECK(ctx_malloc(c, &c->stats_part, (long)kNS * kRedBlocks * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, &c->stats_out, kNS * sizeof(double)));
     const paris_grid_desc& d = c->d;
     StatsArgs a;
     a.u = c->fld[PARIS_FIELD_U]; a.v = c->fld[PARIS_FIELD_V]; a.w = c->fld[PARIS_FIELD_W];

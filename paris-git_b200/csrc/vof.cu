@@ -287,11 +287,10 @@ __global__ void k_c_mask(const double* __restrict__ c, uint8_t* __restrict__ cg,
 // ghost layer, which holds the flux domain of each direction)
 int vof_scratch(paris_ctx* c) {
     const Layout& L = c->L;
-    if (c->vflux) return PARIS_OK;
     const long F = (long)(L.n[0] + 2) * (L.n[1] + 2) * (L.n[2] + 2);
-    PARIS_CUDA_TRY(c, cudaMalloc(&c->vflux, 3 * L.total * sizeof(double)));
-    PARIS_CUDA_TRY(c, cudaMalloc(&c->mixlist, F * sizeof(long)));
-    PARIS_CUDA_TRY(c, cudaMalloc(&c->mixsegn, sizeof(int)));
+    PARIS_CHECK(ctx_malloc(c, &c->vflux, 3 * L.total * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, &c->mixlist, F * sizeof(long)));
+    PARIS_CHECK(ctx_malloc(c, &c->mixsegn, sizeof(int)));
     c->mixcap = F;
     return PARIS_OK;
 }
@@ -373,7 +372,7 @@ extern "C" int paris_vof_sweeps(paris_handle_t c, int32_t tswap, double dt) {
     }
     cudaSetDevice(c->dev);
     if (c->d.vof_advect == PARIS_ADVECT_WY) {
-        if (!c->cg) PARIS_CUDA_TRY(c, cudaMalloc(&c->cg, c->L.total));
+        PARIS_CHECK(ctx_malloc(c, &c->cg, c->L.total));
         PARIS_LAUNCH(c, k_c_mask, div_up(c->L.total, 256), 256, 0, c->fld[PARIS_FIELD_CVOF], c->cg, c->L.total);
     }
     int order[3];
@@ -610,13 +609,16 @@ extern "C" int paris_init_spheres(paris_handle_t c, int32_t nb, const double* xc
         }
     cudaSetDevice(c->dev);
     double* dbuf = nullptr;
-    PARIS_CUDA_TRY(c, cudaMalloc(&dbuf, 4L * nb * sizeof(double)));
+    PARIS_CHECK(ctx_malloc(c, &dbuf, 4L * nb * sizeof(double)));
     const double* src[4] = {xc, yc, zc, rad};
     for (int q = 0; q < 4; q++)
         PARIS_CUDA_TRY(c, cudaMemcpyAsync(dbuf + q * nb, src[q], nb * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     Spheres S{dbuf, dbuf + nb, dbuf + 2 * nb, dbuf + 3 * nb, nb};
     int8_t* f2 = nullptr;
-    PARIS_CUDA_TRY(c, cudaMalloc(&f2, c->L.total));
+    if (ctx_malloc(c, &f2, c->L.total) != PARIS_OK) {
+        cudaFree(dbuf);
+        return PARIS_CUDA_ERROR;
+    }
     PARIS_CUDA_TRY(c, cudaMemsetAsync(f2, 0, c->L.total, c->stream));
     dim3 grid(div_up(c->L.n[0], 64), c->L.n[1], c->L.n[2]);
     long G = ghost_count(c->L);
