@@ -12,7 +12,8 @@
  *     coarse correction (symmetric cycle), coarsest level smoothed; with a
  *     relaxation factor w != 1 each update is x + w (x_GS - x) (the
  *     reference's BETA of RedBlackRelax, newsolver.f90:229), optionally
- *     another factor on the levels below the finest; optionally
+ *     another factor on the levels below the finest; same-coloured neighbours
+ *     over an odd periodic seam (coarsest level) as before the pass; optionally
  *     nu_coarse sweeps each way on the levels coarse_from..coarse_to;
  *   - an FP64 outer loop: defect correction p += V(b - A p), or
  *     preconditioned CG with the V-cycle as preconditioner, with A applied
@@ -26,6 +27,7 @@
  */
 #include <math.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 #include "og.h"
 
@@ -80,6 +82,13 @@ static inline int wrapm(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n :
 #define DEF_OPS(T, SUF, CX, CY, CZ)                                                          \
 static void smooth_##SUF(const fm_mg* mg, fm_level* l, const T* b, T* x, int color) {        \
     const int* per = mg->per;                                                                \
+    /* a periodic axis with an odd extent joins cells of one colour, its first and its last: */ \
+    /* they are taken as they were before the pass, and the diagonal is raised where that    */ \
+    /* could make an over-relaxed pass grow                                                  */ \
+    int seam[3], any = 0;                                                                    \
+    for (int a = 0; a < 3; a++) any += seam[a] = per[a] && l->n[a] % 2;                      \
+    T* old = x;                                                                              \
+    if (any) { old = malloc(l->N * sizeof(T)); memcpy(old, x, l->N * sizeof(T)); }           \
     for (int k = 0; k < l->n[2]; k++)                                                        \
         for (int j = 0; j < l->n[1]; j++)                                                    \
             for (int i = (j + k + color) & 1; i < l->n[0]; i += 2) {                         \
@@ -88,19 +97,29 @@ static void smooth_##SUF(const fm_mg* mg, fm_level* l, const T* b, T* x, int col
                 T a3 = FM_WEST(l, per, l->CY, i, j, k, 1), a4 = l->CY[q];                    \
                 T a5 = FM_WEST(l, per, l->CZ, i, j, k, 2), a6 = l->CZ[q];                    \
                 T pw, pe, ps, pn, pb, pt;                                                    \
-                FM_NBR(T, l, per, x, i, j, k, -1, 0, 0, pw);                                 \
-                FM_NBR(T, l, per, x, i, j, k, 1, 0, 0, pe);                                  \
-                FM_NBR(T, l, per, x, i, j, k, 0, -1, 0, ps);                                 \
-                FM_NBR(T, l, per, x, i, j, k, 0, 1, 0, pn);                                  \
-                FM_NBR(T, l, per, x, i, j, k, 0, 0, -1, pb);                                 \
-                FM_NBR(T, l, per, x, i, j, k, 0, 0, 1, pt);                                  \
+                FM_NBR(T, l, per, old, i, j, k, -1, 0, 0, pw);                               \
+                FM_NBR(T, l, per, old, i, j, k, 1, 0, 0, pe);                                \
+                FM_NBR(T, l, per, old, i, j, k, 0, -1, 0, ps);                               \
+                FM_NBR(T, l, per, old, i, j, k, 0, 1, 0, pn);                                \
+                FM_NBR(T, l, per, old, i, j, k, 0, 0, -1, pb);                               \
+                FM_NBR(T, l, per, old, i, j, k, 0, 0, 1, pt);                                \
                 T d = a1 + a2 + a3 + a4 + a5 + a6;                                           \
-                T s = a1 * pw + a2 * pe + a3 * ps + a4 * pn + a5 * pb + a6 * pt + b[q];       \
+                T s = a1 * pw + a2 * pe + a3 * ps + a4 * pn + a5 * pb + a6 * pt + b[q];      \
                 if (d > (T)0) {                                                              \
-                    const T g = s / d, w = (T)l->omega;                                      \
-                    x[q] = w == (T)1 ? g : x[q] + w * (g - x[q]);                            \
+                    const T w = (T)l->omega;                                                 \
+                    T g = s / d;                                                             \
+                    if (any) {                                                               \
+                        T e = 0;   /* the coefficients over seams */                         \
+                        if (seam[0]) e += i == 0 ? a1 : (i == l->n[0] - 1 ? a2 : (T)0);      \
+                        if (seam[1]) e += j == 0 ? a3 : (j == l->n[1] - 1 ? a4 : (T)0);      \
+                        if (seam[2]) e += k == 0 ? a5 : (k == l->n[2] - 1 ? a6 : (T)0);      \
+                        const T m = (T)0.5 * w * (d + e), up = m > d ? m - d : (T)0;         \
+                        g = (s + up * old[q]) / (d + up);                                    \
+                    }                                                                        \
+                    x[q] = w == (T)1 ? g : old[q] + w * (g - old[q]);                        \
                 }                                                                            \
             }                                                                                \
+    if (any) free(old);                                                                      \
 }                                                                                            \
 /* r = b - A x */                                                                            \
 static void resid_##SUF(const fm_mg* mg, fm_level* l, const T* b, const T* x, T* r) {        \

@@ -303,8 +303,8 @@ extern "C" int paris_gpu_finalize(paris_handle_t c) {
     if (c->s_d2h) cudaStreamDestroy(c->s_d2h);
     for (auto& l : c->ref) { free_ptr(l.K); free_ptr(l.p); free_ptr(l.e); free_ptr(l.q); }
     mg_fast_free_maps(c);
-    for (auto& l : c->fl32) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); }
-    for (auto& l : c->fl64) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); }
+    for (auto& l : c->fl32) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); free_ptr(l.y); }
+    for (auto& l : c->fl64) { free_ptr(l.cx); free_ptr(l.cy); free_ptr(l.cz); free_ptr(l.b); free_ptr(l.x); free_ptr(l.x2); free_ptr(l.y); }
     if (c->red_host) cudaFreeHost(c->red_host);
     if (c->err_host) cudaFreeHost(c->err_host);
     for (auto e : c->evpool) cudaEventDestroy(e);

@@ -35,6 +35,7 @@ struct FastLevel {
     T *cx = nullptr, *cy = nullptr, *cz = nullptr;
     T *b = nullptr, *x = nullptr;
     T* x2 = nullptr;   // second iterate of the fused sweeps (they read one and write the other)
+    T* y = nullptr;    // a coarsest level with an odd periodic axis: second array of its colour passes
     void* tma = nullptr;   // FP32: tensor maps of the level for the TMA-staged sweep (mg_fast.cu)
     bool pairs = false;    // two consecutive sweeps run as one pass (k_rb_sweep4_cfg)
     bool rs = false;       // the last pre-smoothing sweep forms the coarse right-hand side (k_rb_sweep_rs)

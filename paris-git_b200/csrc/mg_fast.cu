@@ -86,59 +86,64 @@ __device__ inline void smooth_cell(const LV<T>& v, const Bnd& B, int i, int j, i
 }
 
 // A periodic axis with an odd number of cells (on the coarsest level only)
-// joins cells of one colour: its first and its last.  A pass over them all at
-// once would read values that it is writing; so a colour pass takes the cells
-// in no such last plane first, then those in one, in two and in three.  Two
-// neighbours of one colour differ by one in that count, and the last plane
-// comes after the first as in the loop order i, j, k: the pass in that order,
-// to the bit.
-__device__ inline int seam_count(const Bnd& B, int n0, int n1, int n2, int i, int j, int k) {
-    return (B.per[0] && (n0 & 1) && i == n0 - 1) + (B.per[1] && (n1 & 1) && j == n1 - 1) +
-           (B.per[2] && (n2 & 1) && k == n2 - 1);
-}
+// joins cells of one colour over its seam: its first and its last.  A colour
+// pass over such a level takes those neighbours as they were before the pass
+// (each colour's values lie in one of two arrays; the pass reads one and writes
+// the other), so no cell reads what the pass writes and any order gives the same
+// bits.  The cells of the colour then relax as in Jacobi's method, which an
+// over-relaxed pair of cells that see little but each other can make grow: the
+// diagonal d is raised to max(d, w (d + e) / 2), e the coefficients over the
+// seam, which keeps 2 D / w - A diagonally dominant and the pass a contraction
+// for every w < 2.  Few cells are raised: w = 1.25 takes e > 0.6 d.  (In loop
+// order, in up to three further passes over the last planes, a solve takes the
+// same iterations within one, but a coarse cycle of 15x9x21 FP64 took 244 us, of
+// 33x25x15 FP32 by launches 620; here 79 and 234, between walls 68 and 211.)
 __host__ __device__ inline int seam_axes(const Bnd& B, int n0, int n1, int n2) {
     return (B.per[0] && (n0 & 1)) + (B.per[1] && (n1 & 1)) + (B.per[2] && (n2 & 1));
 }
-// f(i, j, k) for the cells of the colour in `count` such planes, dealt to st threads
-template <typename F>
-__device__ inline void for_seam_cells(const Bnd& B, int n0, int n1, int n2, int color, int count, int t0, int st, F f) {
-    const bool s0 = B.per[0] && (n0 & 1), s1 = B.per[1] && (n1 & 1), s2 = B.per[2] && (n2 & 1);
-    const int p0 = s0 ? n1 * n2 : 0, p1 = s1 ? n0 * n2 : 0, p2 = s2 ? n0 * n1 : 0;
-    for (int t = t0; t < p0 + p1 + p2; t += st) {
-        int i, j, k;
-        if (t < p0) {
-            i = n0 - 1; k = t / n1; j = t - k * n1;
-        } else if (t < p0 + p1) {
-            const int q = t - p0;
-            j = n1 - 1; k = q / n0; i = q - k * n0;
-            if (s0 && i == n0 - 1) continue;   // (in the planes before)
-        } else {
-            const int q = t - p0 - p1;
-            k = n2 - 1; j = q / n0; i = q - j * n0;
-            if ((s0 && i == n0 - 1) || (s1 && j == n1 - 1)) continue;
-        }
-        if (((i + j + k + color) & 1) == 0 && seam_count(B, n0, n1, n2, i, j, k) == count) f(i, j, k);
-    }
+// x_new of a cell from the sum s of its neighbours and right-hand side
+template <typename T>
+__device__ inline T relax_seam(T s, T d, T e, T x0, T w) {
+    const T m = (T)0.5 * w * (d + e), up = m > d ? m - d : (T)0;
+    return relax((s + up * x0) / (d + up), x0, w);
 }
 
 // grid (ceil(n/128), n1, n2), block 128: one thread per cell of the colour
-// (SEAM: but those in a last plane of a periodic axis with an odd extent)
-template <typename T, bool SEAM>
+template <typename T>
 __global__ void k_fast_smooth(const LV<T> v, const Bnd B, int color) {
     int ih = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
     int i = 2 * ih + ((j + k + color) & 1);
-    if (i < v.n0 && !(SEAM && seam_count(B, v.n0, v.n1, v.n2, i, j, k))) smooth_cell(v, B, i, j, k);
+    if (i < v.n0) smooth_cell(v, B, i, j, k);
 }
 
-// the rest of a SEAM pass, one block
+// the same on a level with such a seam: the cells of the colour from `same`,
+// the others from `other`, into `out`
 template <typename T>
-__global__ void __launch_bounds__(1024) k_fast_smooth_seam(const LV<T> v, const Bnd B, int color) {
-    const int axes = seam_axes(B, v.n0, v.n1, v.n2);
-    for (int count = 1; count <= axes; count++) {
-        for_seam_cells(B, v.n0, v.n1, v.n2, color, count, threadIdx.x, blockDim.x,
-                       [&](int i, int j, int k) { smooth_cell(v, B, i, j, k); });
-        __syncthreads();
-    }
+__global__ void k_fast_smooth_seam(const LV<T> v, const T* same, const T* other, T* out, const Bnd B, int color) {
+    const int ih = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+    const int i = 2 * ih + ((j + k + color) & 1);
+    if (i >= v.n0) return;
+    const long m = cidx(v.n0, v.n1, i, j, k);
+    const long sy = v.n0, sz = (long)v.n0 * v.n1;
+    T a1, a3, a5;
+    west_coefs(v, B, i, j, k, m, a1, a3, a5);
+    const T a2 = v.cx[m], a4 = v.cy[m], a6 = v.cz[m];
+    T e = (T)0;
+    // the neighbour at m + o, over the periodic end of an axis of n cells at m + w
+    auto nb = [&](bool end, int per, int n, long o, long w, T a) {
+        if (!end) return other[m + o];
+        if (!per) return (T)0;
+        if (n & 1) e += a;
+        return (n & 1 ? same : other)[m + w];
+    };
+    const T x1 = nb(i == 0, B.per[0], v.n0, -1, v.n0 - 1, a1), x2 = nb(i == v.n0 - 1, B.per[0], v.n0, 1, 1 - v.n0, a2);
+    const T x3 = nb(j == 0, B.per[1], v.n1, -sy, sy * (v.n1 - 1), a3);
+    const T x4 = nb(j == v.n1 - 1, B.per[1], v.n1, sy, -sy * (v.n1 - 1), a4);
+    const T x5 = nb(k == 0, B.per[2], v.n2, -sz, sz * (v.n2 - 1), a5);
+    const T x6 = nb(k == v.n2 - 1, B.per[2], v.n2, sz, -sz * (v.n2 - 1), a6);
+    const T d = a1 + a2 + a3 + a4 + a5 + a6;
+    const T s = a1 * x1 + a2 * x2 + a3 * x3 + a4 * x4 + a5 * x5 + a6 * x6 + v.b[m];
+    out[m] = d > (T)0 ? relax_seam(s, d, e, same[m], v.omega) : same[m];
 }
 
 // Residual and restriction with one warp per 32 coarse cells of a fine row:
@@ -270,12 +275,13 @@ __device__ inline CcNb cc_nb(const CcLvl& l, const Bnd& B, int i, int j, int k) 
     return q;
 }
 
+// x1..x6: the indices of the neighbours' values
 template <typename T>
-__device__ inline void cc_terms(const T* sm, const CcLvl& l, const CcNb& q, T& a1, T& a2, T& a3, T& a4, T& a5, T& a6,
-                                T& xw, T& xe, T& xs, T& xn, T& xb, T& xt) {
-    const T* x = sm + l.x;
+__device__ inline void cc_terms(const T* sm, const CcLvl& l, const CcNb& q, int x1, int x2, int x3, int x4, int x5,
+                                int x6, T& a1, T& a2, T& a3, T& a4, T& a5, T& a6, T& xw, T& xe, T& xs, T& xn, T& xb,
+                                T& xt) {
     const T c1 = sm[l.cx + q.mw], c3 = sm[l.cy + q.ms], c5 = sm[l.cz + q.mb];
-    const T vw = x[q.mw], ve = x[q.me], vs = x[q.ms], vn = x[q.mn], vb = x[q.mb], vt = x[q.mt];
+    const T vw = sm[x1], ve = sm[x2], vs = sm[x3], vn = sm[x4], vb = sm[x5], vt = sm[x6];
     a1 = q.hw ? c1 : (T)0;
     a3 = q.hs ? c3 : (T)0;
     a5 = q.hb ? c5 : (T)0;
@@ -290,9 +296,9 @@ __device__ inline void cc_terms(const T* sm, const CcLvl& l, const CcNb& q, T& a
     a6 = sm[l.cz + q.m];
 }
 
-// SEAM: the coarsest level has a periodic axis with an odd extent (a kernel of
-// its own: in one, the further passes took registers from all, 58 to 117 us for the
-// FP64 cycle of 16^3 cells)
+// SEAM: the coarsest level has a periodic axis with an odd extent (k_fast_smooth_seam;
+// its second array lies behind the scratch array).  A kernel of its own: in one,
+// what it holds takes registers from all levels.
 template <typename T, bool SEAM>
 __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, int L0, int nl, const Bnd B, int nu1,
                                                             int nu2, int nuc, int cf, int ct, int scratch) {
@@ -346,35 +352,46 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
         if (warp) __syncwarp();
         else __syncthreads();
     };
-    auto update = [&](const CcLvl& l, T w, int i, int j, int k) {
-        const CcNb q = cc_nb(l, B, i, j, k);
-        T a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt;
-        cc_terms(sm, l, q, a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt);
-        T d = a1 + a2 + a3 + a4 + a5 + a6;
-        T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + sm[l.b + q.m];
-        T* x = sm + l.x;
-        if (d > (T)0) x[q.m] = relax(s / d, w != (T)1 ? x[q.m] : (T)0, w);
-    };
-    // one colour pass of red-black Gauss-Seidel over level l
-    auto smooth = [&](const CcLvl& l, T w, int color, bool warp) {
-        const int axes = SEAM ? seam_axes(B, l.n0, l.n1, l.n2) : 0;   // (none but on the coarsest)
+    // one colour pass of red-black Gauss-Seidel over level l; with `at`, one over
+    // the coarsest level with its seams: colour c lies in the array at at[c]
+    auto smooth = [&](const CcLvl& l, T w, int color, bool warp, int* at) {
         const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
         const int h0 = (l.n0 + 1) >> 1, hn = h0 * l.n1;
         const int tot = hn * l.n2;
         const float rhn = 1.0f / (float)hn, rh0 = 1.0f / (float)h0;
+        const bool s0 = B.per[0] && (l.n0 & 1), s1 = B.per[1] && (l.n1 & 1), s2 = B.per[2] && (l.n2 & 1);
+        int same = l.x, other = l.x, out = l.x;
+        if (SEAM && at) {
+            same = at[color];
+            other = at[1 - color];
+            out = same == l.x ? scratch + (L0 < nl - 1 ? S[L0].N : 0) : l.x;
+        }
         for (int t = t0; t < tot; t += st) {
             const int k = div_small(t, hn, rhn), r = t - k * hn;
             const int j = div_small(r, h0, rh0), ih = r - j * h0;
             const int i = 2 * ih + ((j + k + color) & 1);
-            if (i >= l.n0 || (SEAM && seam_count(B, l.n0, l.n1, l.n2, i, j, k))) continue;
-            update(l, w, i, j, k);
+            if (i >= l.n0) continue;
+            const CcNb q = cc_nb(l, B, i, j, k);
+            T a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt;
+            const bool w1 = SEAM && at && s0 && i == 0, w2 = SEAM && at && s0 && i == l.n0 - 1;
+            const bool w3 = SEAM && at && s1 && j == 0, w4 = SEAM && at && s1 && j == l.n1 - 1;
+            const bool w5 = SEAM && at && s2 && k == 0, w6 = SEAM && at && s2 && k == l.n2 - 1;
+            cc_terms(sm, l, q, (w1 ? same : other) + q.mw, (w2 ? same : other) + q.me, (w3 ? same : other) + q.ms,
+                     (w4 ? same : other) + q.mn, (w5 ? same : other) + q.mb, (w6 ? same : other) + q.mt, a1, a2, a3, a4,
+                     a5, a6, xw, xe, xs, xn, xb, xt);
+            const T e = (w1 ? a1 : (w2 ? a2 : (T)0)) + (w3 ? a3 : (w4 ? a4 : (T)0)) + (w5 ? a5 : (w6 ? a6 : (T)0));
+            T d = a1 + a2 + a3 + a4 + a5 + a6;
+            T s = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + sm[l.b + q.m];
+            if (SEAM && at) {
+                const T x0 = sm[same + q.m];
+                sm[out + q.m] = d > (T)0 ? relax_seam(s, d, e, x0, w) : x0;
+            } else if (d > (T)0) {
+                T* x = sm + l.x;
+                x[q.m] = relax(s / d, w != (T)1 ? x[q.m] : (T)0, w);
+            }
         }
         sync(warp);
-        for (int count = 1; count <= axes; count++) {
-            for_seam_cells(B, l.n0, l.n1, l.n2, color, count, t0, st,
-                           [&](int i, int j, int k) { update(l, w, i, j, k); });
-            sync(warp);
-        }
+        if (SEAM && at) at[color] = out;
     };
     auto down = [&](int L, bool warp) {   // zero, pre-smooth and restrict level L, or solve the coarsest
         const int t0 = warp ? lane : tid, st = warp ? 32 : nt;
@@ -383,11 +400,12 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
         for (int t = t0; t < l.N; t += st) sm[l.x + t] = (T)0;
         sync(warp);
         if (L == nl - 1) {
-            for (int s = 0; s < kCoarseSweeps; s++) { smooth(l, w, 0, warp); smooth(l, w, 1, warp); }
-            for (int s = 0; s < kCoarseSweeps; s++) { smooth(l, w, 1, warp); smooth(l, w, 0, warp); }
+            int where[2] = {l.x, l.x}, *at = SEAM ? where : nullptr;   // (back in x after an even number of passes)
+            for (int s = 0; s < kCoarseSweeps; s++) { smooth(l, w, 0, warp, at); smooth(l, w, 1, warp, at); }
+            for (int s = 0; s < kCoarseSweeps; s++) { smooth(l, w, 1, warp, at); smooth(l, w, 0, warp, at); }
             return;
         }
-        for (int s = 0; s < nu_at(L, nu1, nuc, cf, ct); s++) { smooth(l, w, 0, warp); smooth(l, w, 1, warp); }
+        for (int s = 0; s < nu_at(L, nu1, nuc, cf, ct); s++) { smooth(l, w, 0, warp, nullptr); smooth(l, w, 1, warp, nullptr); }
         // residuals of the fine cells into the scratch array
         {
             const int fn = l.n0 * l.n1;
@@ -397,7 +415,8 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
                 const int j = div_small(r, l.n0, rf0), i = r - j * l.n0;
                 const CcNb q = cc_nb(l, B, i, j, k);
                 T a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt;
-                cc_terms(sm, l, q, a1, a2, a3, a4, a5, a6, xw, xe, xs, xn, xb, xt);
+                cc_terms(sm, l, q, l.x + q.mw, l.x + q.me, l.x + q.ms, l.x + q.mn, l.x + q.mb, l.x + q.mt, a1, a2, a3,
+                         a4, a5, a6, xw, xe, xs, xn, xb, xt);
                 T d = a1 + a2 + a3 + a4 + a5 + a6;
                 sm[scratch + q.m] =
                     sm[l.b + q.m] - d * sm[l.x + q.m] + a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt;
@@ -435,7 +454,7 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
             sm[l.x + t] += sm[c.x + (i >> 1) + c.n0 * ((j >> 1) + c.n1 * (k >> 1))];
         }
         sync(warp);
-        for (int s = 0; s < nu_at(L, nu2, nuc, cf, ct); s++) { smooth(l, w, 1, warp); smooth(l, w, 0, warp); }
+        for (int s = 0; s < nu_at(L, nu2, nuc, cf, ct); s++) { smooth(l, w, 1, warp, nullptr); smooth(l, w, 0, warp, nullptr); }
     };
     int Lw = L0;   // first level worked by warp 0
     while (Lw < nl && S[Lw].N > kWarpCells) Lw++;
@@ -456,8 +475,8 @@ __global__ void __launch_bounds__(1024) k_coarse_cycle_smem(const LVSet<T> G, in
 }
 
 // A coarsest level of more than 16^3 cells still runs in one block where its
-// five arrays fit (11.5 thousand cells FP32, 5.7 FP64), and by launches of colour
-// passes above.  Measured us per V-cycle (of grids four times as wide), one block
+// five arrays (six with a seam) fit, 11.5 thousand cells FP32 and 5.7 FP64 (9.6 and
+// 4.8), and by launches of colour passes above.  Measured us per V-cycle (of grids four times as wide), one block
 // against launches, coarsest level of 17^3 cells 201 / 263 FP32 and 240 / 273
 // FP64, 25x20x15 229 / 265 FP32, 27x21x15 242 / 267 FP32; one block on global
 // memory, which larger ones took before, 346 / 293 at 33x25x15 FP32, 324 / 284 at
@@ -916,6 +935,8 @@ static int fast_levels(paris_ctx* c) {
             PARIS_CHECK(ctx_malloc(c, &l.x2, l.N * sizeof(T)));
             PARIS_CHECK(sweep_col_choose(c, l));
         }
+        if (L == nl - 1 && l.N > kCoarseCells && seam_axes(c->bnd, l.n[0], l.n[1], l.n[2]))
+            PARIS_CHECK(ctx_malloc(c, &l.y, l.N * sizeof(T)));
         l.pairs = fusable && pairs_wanted();
         l.rs = fusable && std::is_same<T, float>::value && (rs_levels() == 2 || (rs_levels() == 1 && L == 0));
         l.merged = fusable && std::is_same<T, float>::value ? merged_wanted() : 0;
@@ -933,7 +954,7 @@ static int fast_alloc(paris_ctx* c) {
     if (st != PARIS_OK) {
         if (std::is_same<T, float>::value) mg_fast_free_maps(c);
         for (FastLevel<T>& l : lv) {
-            T* const all[] = {l.cx, l.cy, l.cz, l.b, l.x, l.x2};
+            T* const all[] = {l.cx, l.cy, l.cz, l.b, l.x, l.x2, l.y};
             for (T* p : all) cudaFree(p);
         }
         lv.clear();
@@ -1143,8 +1164,8 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_CUDA_TRY(c, cudaMemsetAsync(l.x, 0, l.N * sizeof(T), c->stream));
             LV<T> v = view(l);
             for (int s = 0; s < nu1; s++) {
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
             }
             cur[L] = l.x;
         }
@@ -1153,30 +1174,33 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_LAUNCH_N(c, kname<T>("mg_restrict"), l.N, k_fast_restrict2<T>,
                            dim3(div_up(cv.n0, 32), cv.n1, cv.n2), dim3(32, 4), 0, view_x(l, cur[L]), cv, c->bnd);
     }
-    if (coarse_smem(lv, Lc) > kBlockSmem) {   // the coarsest, too large for a block
-        const LV<T> v = view(lv[Lc]);
+    // from 16^3 down, the levels, a scratch array of the largest restricted one and
+    // the second array of a coarsest level with seams fit the shared memory (at most
+    // 223 KB, FP64)
+    const FastLevel<T>& last = lv[nl - 1];
+    const bool seam = seam_axes(c->bnd, last.n[0], last.n[1], last.n[2]) > 0;
+    const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
+    const size_t csm = (scratch + (Lc < nl - 1 ? lv[Lc].N : 0) + (seam ? last.N : 0)) * sizeof(T);
+    if (csm > kBlockSmem) {   // the coarsest, too large for a block
+        const LV<T> v = view(last);
         PARIS_CUDA_TRY(c, cudaMemsetAsync(v.x, 0, v.N * sizeof(T), c->stream));
-        const bool seam = seam_axes(c->bnd, v.n0, v.n1, v.n2) > 0;
         const dim3 grid = row_grid((v.n0 + 1) / 2, v.n1, v.n2);
+        T* at[2] = {v.x, v.x};   // the array of each colour; back in x after an even number of passes
         for (int s = 0; s < 4 * kCoarseSweeps; s++) {
             const int color = s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1);
             if (seam) {
-                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, (k_fast_smooth<T, true>), grid, 128, 0, v, c->bnd, color);
-                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), 0L, k_fast_smooth_seam<T>, 1, 1024, 0, v, c->bnd, color);
+                T* const out = at[color] == v.x ? last.y : v.x;
+                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, k_fast_smooth_seam<T>, grid, 128, 0, v, at[color],
+                               at[1 - color], out, c->bnd, color);
+                at[color] = out;
             } else {
-                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, (k_fast_smooth<T, false>), grid, 128, 0, v, c->bnd, color);
+                PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), v.N, k_fast_smooth<T>, grid, 128, 0, v, c->bnd, color);
             }
         }
     } else {
         LVSet<T> S;
         for (int L = 0; L < nl; L++) S.l[L] = view(lv[L]);
-        // from 16^3 down, the levels and a scratch array of the largest restricted
-        // one fit the shared memory (at most 219 KB, FP64)
-        const size_t scratch = coarse_smem(lv, Lc) / sizeof(T);
-        const size_t csm = coarse_smem(lv, Lc) + (Lc < nl - 1 ? (size_t)lv[Lc].N * sizeof(T) : 0);
-        const FastLevel<T>& last = lv[nl - 1];
-        auto* const kern = seam_axes(c->bnd, last.n[0], last.n[1], last.n[2]) ? &k_coarse_cycle_smem<T, true>
-                                                                              : &k_coarse_cycle_smem<T, false>;
+        auto* const kern = seam ? &k_coarse_cycle_smem<T, true> : &k_coarse_cycle_smem<T, false>;
         if (!ctx_kernel_blocks(c, (const void*)kern, 1024, csm)) return PARIS_CUDA_ERROR;
         PARIS_LAUNCH_N(c, kname<T>("mg_coarse_cycle"), lv[Lc].N, kern, 1, 1024, csm, S, Lc, nl, c->bnd, nu1_, nu2_, nuc,
                        cf, ct, (int)scratch);
@@ -1210,8 +1234,8 @@ static int vcycle(paris_ctx* c, int nu1_, int nu2_, T** x0) {
             PARIS_LAUNCH_N(c, kname<T>("mg_prolong"), v.N, k_fast_prolong<T>, row_grid(v.n0, v.n1, v.n2), 128, 0, v,
                            view_x(lv[L + 1], cur[L + 1]));
             for (int s = 0; s < nu2; s++) {
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
-                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, (k_fast_smooth<T, false>), row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 1);
+                PARIS_LAUNCH_N(c, kname<T>("mg_smooth"), v.N, k_fast_smooth<T>, row_grid((v.n0 + 1) / 2, v.n1, v.n2), 128, 0, v, c->bnd, 0);
             }
         }
     }

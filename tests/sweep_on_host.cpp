@@ -52,6 +52,29 @@ static void pass(const LV<T>& v, const Bnd& B, int color, bool sweep) {
             }
 }
 
+// the same on a level with odd periodic seams: from the values before the pass
+template <typename T>
+static void pass_seam(const LV<T>& v, const Bnd& B, int color) {
+    const std::vector<T> old(v.x, v.x + v.N);
+    const bool s[3] = {B.per[0] && v.n0 % 2, B.per[1] && v.n1 % 2, B.per[2] && v.n2 % 2};
+    for (int k = 0; k < v.n2; k++)
+        for (int j = 0; j < v.n1; j++)
+            for (int i = (j + k + color) & 1; i < v.n0; i += 2) {
+                const long m = cidx(v.n0, v.n1, i, j, k);
+                T a1, a3, a5, xw, xe, xs, xn, xb, xt, e = 0;
+                west_coefs(v, B, i, j, k, m, a1, a3, a5);
+                const T a2 = v.cx[m], a4 = v.cy[m], a6 = v.cz[m];
+                nbrs(v, old.data(), B, i, j, k, m, xw, xe, xs, xn, xb, xt);
+                if (s[0]) e += i == 0 ? a1 : (i == v.n0 - 1 ? a2 : (T)0);
+                if (s[1]) e += j == 0 ? a3 : (j == v.n1 - 1 ? a4 : (T)0);
+                if (s[2]) e += k == 0 ? a5 : (k == v.n2 - 1 ? a6 : (T)0);
+                const T d = a1 + a2 + a3 + a4 + a5 + a6;
+                const T sum = a1 * xw + a2 * xe + a3 * xs + a4 * xn + a5 * xb + a6 * xt + v.b[m];
+                const T up = (T)0.5 * v.omega * (d + e) > d ? (T)0.5 * v.omega * (d + e) - d : (T)0;
+                if (d > 0) v.x[m] = relax((sum + up * old[m]) / (d + up), old[m], v.omega);
+            }
+}
+
 template <typename T>
 static int same(const T* a, const T* b, long N, const char* what) {
     for (long m = 0; m < N; m++)
@@ -110,21 +133,29 @@ static int run_coarse(const int* n, const int* per, int nl, unsigned threads) {
     if (nl > 1) return 0;   // (races only)
     std::vector<T> ref(S.l[0].N, (T)0);
     const LV<T> r = p[0]->view(ref.data(), (T)1.1);
-    for (int s = 0; s < 4 * kCoarseSweeps; s++) pass(r, p[0]->B, s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1), false);
+    const bool seam = seam_axes(p[0]->B, r.n0, r.n1, r.n2) > 0;
+    for (int s = 0; s < 4 * kCoarseSweeps; s++) {
+        const int color = s < 2 * kCoarseSweeps ? s & 1 : 1 - (s & 1);
+        if (seam) pass_seam(r, p[0]->B, color);
+        else pass(r, p[0]->B, color, false);
+    }
     return same(p[0]->x, ref.data(), r.N, "coarse cycle");
 }
 
-// colour passes over a whole level by launches, two passes
+// colour passes over a whole level by launches, four of them
 template <typename T>
 static int run_passes(const int* n, const int* per) {
     Problem<T> p(n[0], n[1], n[2], per);
     const LV<T> v = p.view(p.x, (T)1.1);
     std::vector<T> ref(p.x, p.x + v.N);
     const LV<T> r = p.view(ref.data(), (T)1.1);
-    for (int color = 0; color < 2; color++) {
-        launch(dim3(1, n[1], n[2]), 32, [&] { k_fast_smooth<T, true>(v, p.B, color); });
-        launch(dim3(1), 64, [&] { k_fast_smooth_seam<T>(v, p.B, color); });
-        pass(r, p.B, color, false);
+    T* at[2] = {p.x, p.x};
+    for (int q = 0; q < 4; q++) {
+        const int color = q & 1;
+        T* const out = at[color] == p.x ? p.x2 : p.x;
+        launch(dim3(1, n[1], n[2]), 32, [&] { k_fast_smooth_seam<T>(v, at[color], at[1 - color], out, p.B, color); });
+        at[color] = out;
+        pass_seam(r, p.B, color);
     }
     return same(p.x, ref.data(), v.N, "colour passes");
 }

@@ -1,6 +1,6 @@
 """Coarsest levels that are no power of two, against the CPU oracle's cycle:
-relaxed in one block (up to 5.7 thousand cells FP64, 11.5 FP32) and by launches
-(above), with odd extents over periodic seams, where the first and the last cell
+relaxed in one block (up to 5.7 thousand cells FP64, 11.5 FP32; 4.8 and 9.6 with a
+seam) and by launches (above), with odd extents over periodic seams, where the first and the last cell
 of a row share a colour, and between walls."""
 import warnings
 
@@ -8,13 +8,14 @@ import numpy as np
 import pytest
 
 from sweep_case import problem as _problem
+from test_oracle_fastmg import seam_pairs
 
 pytestmark = pytest.mark.gpu
 
 
-# coarsest levels 5x3x7, 9x10x11, 15x9x21 and 18x17x17 in one block, 25x17x21 in
-# one block (FP32) and by launches (FP64), 27x26x13 likewise, 33x25x15 by launches,
-# 45x23x27 (the whole grid) with no level above it
+# coarsest levels 5x3x7, 9x10x11 and 15x9x21 in one block, 18x17x17, 25x17x21 and
+# 27x26x13 in one block (FP32, and 18x17x17 between walls) and by launches (FP64),
+# 33x25x15 by launches, 45x23x27 (the whole grid) with no level above it
 GRIDS = [((20, 12, 28), "periodic"), ((36, 40, 44), (1, 0, 1, 1, 0, 1)), ((60, 36, 84), "wall"),
          ((60, 36, 84), "periodic"), ((36, 34, 34), "periodic"), ((36, 34, 34), "wall"), ((50, 34, 42), "periodic"),
          ((54, 52, 26), (0, 1, 1, 0, 1, 1)), ((50, 34, 42), "wall"), ((66, 50, 30), "periodic"),
@@ -53,6 +54,22 @@ def test_cycles_follow_oracle(gpu_lib, capi, runtime, orc, workloads, n, bc, mod
     assert np.array_equal(out[0], out[1])
     assert np.abs(d).max() <= tol * np.abs(ref).max()
     assert abs(r.rel_res - hist[-1]) <= 10 * tol * hist[-1]
+
+
+@pytest.mark.parametrize("omega", [1.0, 1.25, 1.5])
+def test_pairs_over_an_odd_seam(gpu_lib, capi, runtime, orc, omega):
+    """Light cells of one colour facing each other over a seam: the solver follows
+    the oracle's CG within one iteration."""
+    desc, rho, vel, A = seam_pairs(capi, orc)
+    _, it, _ = orc.fastmg_solve(desc, A, np.zeros((9, 9, 9)), 1e-10, maxit=100, mixed=False, pcg=True, omega=omega)
+    with runtime.ParisGpu(desc) as gpu:
+        gpu.upload(capi.F_RHO, rho)
+        for f, a in zip((capi.F_U, capi.F_V, capi.F_W), vel):
+            gpu.upload(f, a)
+        gpu.setup_poisson(1e-3)
+        gpu.fill_field(capi.F_P, 0.0)
+        r = gpu.new_solver(0.0, maxit=100, mode=capi.MG_FP64, rel_tol=1e-10, pcg=1, beta=omega)
+    assert r.rel_res < 1e-10 and abs(r.it - it) <= 1
 
 
 def test_handles_in_threads(gpu_lib, capi, runtime, orc, workloads):
