@@ -42,10 +42,9 @@ def scale(d, ab):
     return s
 
 
-@pytest.mark.parametrize("grid", ["general", "pow2"])
 @pytest.mark.parametrize("bc", ["wall", "periodic"])
 @pytest.mark.parametrize("flags", [0, 1, 6])
-def test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags, grid):
+def test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags, grid="general"):
     d, f = state(capi, orc, bc, 5, grid)
     o = capi.make_stats_opts(dpdx=(0.2, -0.1, 0.05), gravity=(0.0, -9.81, 0.3), buoyancy=3, rho_ave=400.0,
                              test_flags=flags)
@@ -64,6 +63,12 @@ def test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags, grid):
     assert out[16] == ref[16] and out[17] == ref[17]            # point values
     assert out[24] == ref[24] == np.count_nonzero(orc.interior(d, f["flag"]) == 2)
     assert out[18] > 0 and out[21] > 0 and out[22] > 0
+
+
+@pytest.mark.parametrize("bc", ["wall", "periodic"])
+@pytest.mark.parametrize("flags", [0, 1, 6])
+def test_calc_stats_with_exact_reciprocals(gpu_lib, capi, runtime, orc, bc, flags):
+    test_calc_stats_follow_oracle(gpu_lib, capi, runtime, orc, bc, flags, grid="pow2")
 
 
 def test_time_step_size_and_cfl_bitwise(gpu_lib, capi, runtime, orc):
